@@ -951,98 +951,4 @@ __global__ void __launch_bounds__(BLOCK, MINB) blk_kernel(AsmParams p) {
     }
 }
 
-// ---- one persistent launch for an uneven batch ------------------------------
-//
-// Ragged stencils in CSR form, each with its own size k_s = ia[s+1] - ia[s],
-// degree P_s (degree[s], or P0 for all) and PHS exponent Q_s = phs, or
-// 2 P_s - 1 when phs = 0: the reference's one-grid-over-all-stencils launch
-// (src/rbf_operators.h:197-200,340) for stencils of any mix of shapes. Warps
-// claim stencils from one device work counter. A system of up to NS unknowns
-// is solved in the warp's shared-memory slot; a larger one (up to NG) in the
-// warp's region of a global scratch buffer, which stays in L2. Supported:
-// P_s in 1..4 and Q_s in {3, 5, 7, 9}; a stencil outside that (or above NG
-// unknowns, or with no neighbour) sets *err and is skipped.
-
-// Runtime-Q dispatch of the fill (the elimination does not depend on P or Q).
-template <typename T, int LDS, int NRHS, int P>
-__device__ __forceinline__ void fill_system_q(const AsmParams& p, int Q, T* S, const double* cx,
-                                              const double* cy, int ks, int e, int lane) {
-    switch (Q) {
-        case 3: fill_system<T, LDS, NRHS, P, 3>(p, S, cx, cy, ks, e, lane); break;
-        case 5: fill_system<T, LDS, NRHS, P, 5>(p, S, cx, cy, ks, e, lane); break;
-        case 7: fill_system<T, LDS, NRHS, P, 7>(p, S, cx, cy, ks, e, lane); break;
-        default: fill_system<T, LDS, NRHS, P, 9>(p, S, cx, cy, ks, e, lane); break;
-    }
-}
-
-// One stencil in the working set `base` (layout L): gather, fill, eliminate,
-// back-substitute, scatter.
-template <typename T, class L, int NRHS, int PB>
-__device__ __forceinline__ void assemble_any(const AsmParams& p, int s, int off, int ks, int P,
-                                             int Q, char* base, int lane) {
-    constexpr int LDS = L::LDS, G = L::G;
-    double* cx = reinterpret_cast<double*>(base + L::off_cx);
-    double* cy = reinterpret_cast<double*>(base + L::off_cy);
-    T* S = reinterpret_cast<T*>(base + L::off_s);
-    int* piv = reinterpret_cast<int*>(base + L::off_piv);
-    int* act = reinterpret_cast<int*>(base + L::off_act);
-    unsigned char* alive = reinterpret_cast<unsigned char*>(base + L::off_alive);
-    const int np = npoly(P), n = np + ks;
-    const int e = gather_scale<L::KMAX, false>(p, off, ks, p.x[s], p.y[s], cx, cy, lane);
-    switch (P) {
-        case 1: fill_system_q<T, LDS, NRHS, 1>(p, Q, S, cx, cy, ks, e, lane); break;
-        case 2: fill_system_q<T, LDS, NRHS, 2>(p, Q, S, cx, cy, ks, e, lane); break;
-        case 3: fill_system_q<T, LDS, NRHS, 3>(p, Q, S, cx, cy, ks, e, lane); break;
-        default: fill_system_q<T, LDS, NRHS, 4>(p, Q, S, cx, cy, ks, e, lane); break;
-    }
-    __syncwarp(group_mask(G));
-    T* pinv = reinterpret_cast<T*>(base + L::off_pinv);
-    const int info = eliminate_blocked<T, L::R, LDS, NRHS, PB>(S, pinv, piv, act, alive, n, lane);
-    T xs[L::R][NRHS];
-    back_substitute_blk<T, L::R, LDS, NRHS, G, false>(S, piv, pinv, nullptr, n, lane, xs, NoHook{}, np);
-    scatter_regs<T, L::R, NRHS, G>(p, xs, np, ks, off, e, info, s, lane);
-}
-
-template <typename T, int NS, int NG, int NRHS, int PB>
-struct CsrCfg {
-    using SmemL = BlkLayout<T, NS, NRHS, NS, PB, 32, false>;  // shared-memory slot
-    using GlobL = BlkLayout<T, NG, NRHS, NG, PB, 32, false>;  // global scratch region
-    static constexpr size_t gbytes = (static_cast<size_t>(GlobL::bytes) + 255) & ~size_t(255);
-};
-
-template <typename T, int NS, int NG, int NRHS, int BLOCK, int PB, int MINB = 1>
-__global__ void __launch_bounds__(BLOCK, MINB)
-    blk_csr_kernel(AsmParams p, const int8_t* degree, int P0, int phs, char* gscratch, int* err) {
-    using C = CsrCfg<T, NS, NG, NRHS, PB>;
-    constexpr int G = 32, GPB = BLOCK / G;
-    extern __shared__ __align__(16) char smem_raw[];
-    const int gib = threadIdx.x / 32;
-    const int lane = threadIdx.x % 32;
-    char* slot = smem_raw + gib * C::SmemL::bytes;
-    char* gslot = gscratch + (static_cast<size_t>(blockIdx.x) * GPB + gib) * C::gbytes;
-    const int nitems = p.nitems_dev ? *p.nitems_dev : p.nitems;
-    const int* list = (p.list && p.list_off_dev) ? p.list + *p.list_off_dev : p.list;
-    for (;;) {
-        int it = 0;
-        if (lane == 0) it = atomicAdd(p.work, 1);
-        it = __shfl_sync(0xffffffffu, it, 0);
-        if (it >= nitems) break;
-        const int s = list ? list[it] : p.item_base + it;
-        const int off = p.ia[s], ks = p.ia[s + 1] - off;
-        const int P = degree ? degree[s] : P0;
-        const int Q = phs ? phs : 2 * P - 1;
-        const int n = ks + npoly(P);
-        const bool ok = P >= 1 && P <= 4 && (Q == 3 || Q == 5 || Q == 7 || Q == 9) && ks >= 1 &&
-                        n <= NG;
-        if (!ok) {
-            if (lane == 0) atomicExch(err, 1);
-            continue;
-        }
-        if (n <= NS)
-            assemble_any<T, typename C::SmemL, NRHS, PB>(p, s, off, ks, P, Q, slot, lane);
-        else
-            assemble_any<T, typename C::GlobL, NRHS, PB>(p, s, off, ks, P, Q, gslot, lane);
-    }
-}
-
 }  // namespace rbfb

@@ -76,6 +76,7 @@ struct AsmParams {
     double Lx, Ly;  // periods (<= 0: open axis)
     int scale;
     int nrhs;
+    int plain_ops;            // every column is Laplace, d/dx or d/dy
     int col_op[kMaxRhs];  // RBFB_OP_* of every right-hand-side column
     int col_ic[kMaxRhs];  // interpolation point index of OP_INTERP columns
     const double* xc;

@@ -14,27 +14,28 @@
 //
 // RBFB_BLK_VARIANT(name, T, NMAX, NRHS, P, Q, MIXED, BLOCK, MINB, PB, PF): the
 // blocked shared-memory kernel (asm_blocked.cuh), one warp per stencil, any
-// system size n <= NMAX, panels of PB columns. RBFB_BLK16_VARIANT: the same
-// with half-warp groups, two stencils per warp.
+// system size n <= NMAX, panels of PB columns (the refined form).
+//
+// RBFB_DM_VARIANT(name, NMAX, NRHS, P, Q, NW, GPB, MINB): the FP64 kernel
+// (asm_dmma.cuh), n <= NMAX, NW warps a stencil, GPB stencils a CTA, MINB
+// resident CTAs. The first shape of a class is its default. Measured on the
+// B200, 262,144 stencils (65,536 at degree 4), ms: k = 35 three one-warp
+// stencils a CTA 3.40, four 3.42, one 3.52; k = 21 one a CTA 1.53, four 1.60;
+// k = 64 two warps a stencil 4.09, four 4.13.
 // The build compiles each line as its own translation unit.
-RBFB_VARIANT(f64_p4q7_n64_smem, double, 16, 2, 64, 3, 4, 7, false, 32, 1, true, true)
-RBFB_VARIANT(f64_p4q7_n80_smem, double, 16, 2, 80, 3, 4, 7, false, 32, 1, true, true)
-RBFB_BLK_VARIANT(b64_p3q5_n45_pb8, double, 45, 3, 3, 5, false, 32, 1, 8, true)
-RBFB_BLK_VARIANT(b64_p3q5_n45_pb8x3, double, 45, 3, 3, 5, false, 96, 4, 8, true)
-RBFB_BLK16_VARIANT(b64_p3q5_n45_pb8_h1, double, 45, 3, 3, 5, false, 32, 1, 8, true)
-RBFB_BLK_VARIANT(b64_p3q5_n48_pb8, double, 48, 3, 3, 5, false, 32, 1, 8, true)
-RBFB_BLK_VARIANT(b64_p2q3_n32_pb8, double, 32, 3, 2, 3, false, 32, 1, 8, true)
-RBFB_BLK_VARIANT(b64_p2q3_n32_pb8x4, double, 32, 3, 2, 3, false, 128, 1, 8, true)
-RBFB_BLK_VARIANT(b64_p2q3_n32_r8, double, 32, 8, 2, 3, false, 32, 1, 8, true)
-RBFB_BLK_VARIANT(b64_p4q7_n64_pb8, double, 64, 3, 4, 7, false, 32, 1, 8, true)
-RBFB_BLK_VARIANT(b64_p4q7_n80_pb8, double, 80, 3, 4, 7, false, 32, 1, 8, true)
+RBFB_DM_VARIANT(b64_p2q3_n32_w1x1, 32, 3, 2, 3, 1, 1, 20)
+RBFB_DM_VARIANT(b64_p2q3_n32_w1x4_r8, 32, 8, 2, 3, 1, 4, 4)
+RBFB_DM_VARIANT(b64_p3q5_n45_w1x3, 45, 3, 3, 5, 1, 3, 4)
+RBFB_DM_VARIANT(b64_p3q5_n45_w1x1, 45, 3, 3, 5, 1, 1, 12)
+RBFB_DM_VARIANT(b64_p3q5_n48_w1x3, 48, 3, 3, 5, 1, 3, 3)
+RBFB_DM_VARIANT(b64_p4q7_n64_w1, 64, 3, 4, 7, 1, 1, 6)
+RBFB_DM_VARIANT(b64_p4q7_n64_w2, 64, 3, 4, 7, 2, 1, 6)
+RBFB_DM_VARIANT(b64_p4q7_n80_w2, 80, 3, 4, 7, 2, 1, 4)
+RBFB_DM_VARIANT(b64_p4q7_n80_w4, 80, 3, 4, 7, 4, 1, 4)
 RBFB_BLK_VARIANT(bmx_p3q5_n45_pb8, float, 45, 3, 3, 5, true, 32, 1, 8, true)
 RBFB_BLK_VARIANT(bmx_p3q5_n45_pb8x3, float, 45, 3, 3, 5, true, 96, 1, 8, true)
 RBFB_BLK_VARIANT(bmx_p2q3_n32_pb8, float, 32, 3, 2, 3, true, 32, 1, 8, true)
 RBFB_BLK_VARIANT(bmx_p4q7_n80_pb8, float, 80, 3, 4, 7, true, 32, 1, 8, true)
-RBFB_VARIANT(f64_p2q3_n32_g16x2, double, 16, 2, 32, 3, 2, 3, false, 64, 6, false, true)
-RBFB_VARIANT(f64_p2q3_n32_g16x1, double, 16, 1, 32, 3, 2, 3, false, 64, 1, false, true)
-RBFB_VARIANT(f64_p3q5_n48_g16x2, double, 16, 2, 48, 3, 3, 5, false, 64, 1, false, false)
 RBFB_VARIANT(mix_p2q3_n32_g16x1, float, 16, 1, 32, 3, 2, 3, true, 64, 1, false, true)
 RBFB_VARIANT(mix_p2q3_n32_g16x2, float, 16, 2, 32, 3, 2, 3, true, 64, 1, false, true)
 RBFB_VARIANT(mix_p3q5_n48_g16x2, float, 16, 2, 48, 3, 3, 5, true, 64, 4, false, true)

@@ -5,6 +5,7 @@
 #include <cuda_runtime.h>
 
 #include "asm_blocked.cuh"
+#include "asm_dmma.cuh"
 #include "asm_kernel.cuh"
 #include "asm_variants.h"
 
@@ -34,15 +35,15 @@ Variant make_variant(const char* name) {
 }
 
 template <typename T, int NMAX, int NRHS, int P, int Q, bool MIXED, int BLOCK, int MINB, int PB,
-          bool PF, int GW = 32>
+          bool PF>
 Variant make_blk_variant(const char* name) {
-    using C = BlkCfg<T, NMAX, NRHS, P, Q, MIXED, PB, GW>;
+    using C = BlkCfg<T, NMAX, NRHS, P, Q, MIXED, PB>;
     Variant v{};
     v.name = name;
     v.kernel = reinterpret_cast<const void*>(
-        &blk_kernel<T, NMAX, NRHS, P, Q, MIXED, BLOCK, MINB, PB, PF, GW>);
+        &blk_kernel<T, NMAX, NRHS, P, Q, MIXED, BLOCK, MINB, PB, PF>);
     v.launch = [](dim3 grid, int block, size_t smem, cudaStream_t st, const AsmParams& p) {
-        blk_kernel<T, NMAX, NRHS, P, Q, MIXED, BLOCK, MINB, PB, PF, GW><<<grid, block, smem, st>>>(p);
+        blk_kernel<T, NMAX, NRHS, P, Q, MIXED, BLOCK, MINB, PB, PF><<<grid, block, smem, st>>>(p);
     };
     v.mixed = MIXED;
     v.P = P;
@@ -56,20 +57,40 @@ Variant make_blk_variant(const char* name) {
     return v;
 }
 
+template <int NMAX, int NRHS, int P, int Q, int NW, int GPB, int MINB>
+Variant make_dm_variant(const char* name) {
+    using L = dm::Layout<NMAX, NRHS, NMAX - npoly(P)>;
+    Variant v{};
+    v.name = name;
+    v.kernel = reinterpret_cast<const void*>(&dm::dm_kernel<NMAX, NRHS, P, Q, NW, GPB, MINB>);
+    v.launch = [](dim3 grid, int block, size_t smem, cudaStream_t st, const AsmParams& p) {
+        dm::dm_kernel<NMAX, NRHS, P, Q, NW, GPB, MINB><<<grid, block, smem, st>>>(p);
+    };
+    v.mixed = false;
+    v.P = P;
+    v.Q = Q;
+    v.ntp = NMAX;
+    v.nrhs = NRHS;
+    v.group = 32 * NW;
+    v.block = 32 * NW * GPB;
+    v.smem_group = L::bytes;
+    v.smem_block = L::bytes * GPB;
+    return v;
+}
+
 }  // namespace rbfb
+
+#define RBFB_DEFINE_DM_VARIANT(name, NMAX, NRHS, P, Q, NW, GPB, MINB)                           \
+    namespace rbfb {                                                                           \
+    Variant variant_##name() {                                                                 \
+        return make_dm_variant<NMAX, NRHS, P, Q, NW, GPB, MINB>(#name);                        \
+    }                                                                                          \
+    }
 
 #define RBFB_DEFINE_BLK_VARIANT(name, T, NMAX, NRHS, P, Q, MIXED, BLOCK, MINB, PB, PF)          \
     namespace rbfb {                                                                           \
     Variant variant_##name() {                                                                 \
         return make_blk_variant<T, NMAX, NRHS, P, Q, MIXED, BLOCK, MINB, PB, PF>(#name);       \
-    }                                                                                          \
-    }
-
-// the same with half-warp groups: two stencils per warp
-#define RBFB_DEFINE_BLK16_VARIANT(name, T, NMAX, NRHS, P, Q, MIXED, BLOCK, MINB, PB, PF)        \
-    namespace rbfb {                                                                           \
-    Variant variant_##name() {                                                                 \
-        return make_blk_variant<T, NMAX, NRHS, P, Q, MIXED, BLOCK, MINB, PB, PF, 16>(#name);   \
     }                                                                                          \
     }
 

@@ -1,7 +1,7 @@
 // batch.cu -- uneven stencils: rbfb_assemble_csr.
 //
 // FP64 batches (up to 3 right-hand sides) run as ONE persistent launch of the
-// uneven kernel (asm_blocked.cuh, blk_csr_kernel): warps claim stencils of
+// uneven kernel (asm_dmma.cuh, dm_csr_kernel): warps claim stencils of
 // any size and degree from a device counter, walking a list sorted by class
 // on the device (largest systems first); systems of up to 45 unknowns are
 // solved in shared memory, larger ones (up to 96) in an L2-resident global
@@ -26,7 +26,7 @@
 #include <cstring>
 #include <vector>
 
-#include "asm_blocked.cuh"
+#include "asm_dmma.cuh"
 #include "runtime.h"
 
 namespace rbfb {
@@ -34,13 +34,12 @@ namespace {
 
 // The single-launch FP64 kernel for uneven batches: systems of up to 45
 // unknowns (degree 3 with k = 35, the largest interior stencil in common
-// use) in a 19 KB shared-memory slot, 11 CTAs of one warp per SM; up to 96
-// in global scratch. Its n > 45 body (three list slots a lane) would set
-// the register count of every path (230); bounded to 11 CTAs per SM it fits
-// in 168 registers, spilling only on that rare path.
-constexpr int kOneNS = 45, kOneNG = 96, kOneBlock = 32, kOnePB = 8, kOneMinB = 11;
-using OneCfg = CsrCfg<double, kOneNS, kOneNG, 3, kOnePB>;
-constexpr int kOneSmem = OneCfg::SmemL::bytes * (kOneBlock / 32);
+// use) in a 19 KB shared-memory slot, 4 CTAs of three warps per SM; up to 96
+// in global scratch.
+constexpr int kOneNS = 45, kOneNG = 96, kOneGroups = 3, kOneMinB = 4;
+constexpr int kOneBlock = 32 * kOneGroups;
+using OneCfg = dm::CsrCfg<kOneNS, kOneNG, 3>;
+constexpr int kOneSmem = OneCfg::SmemL::bytes * kOneGroups;
 // The launch walks the stencils sorted by class (system size descending,
 // then degree): warps on one SM then run the same fill and elimination
 // bodies (the instruction cache holds one at a time), and the largest
@@ -206,7 +205,7 @@ int build_table(rbfb_ctx* ctx, BatchState* b, bool mixed, int phs, int Pmin, int
 // stream capture).
 int ensure_one(rbfb_ctx* ctx, BatchState* b) {
     const void* k = reinterpret_cast<const void*>(
-        &blk_csr_kernel<double, kOneNS, kOneNG, 3, kOneBlock, kOnePB, kOneMinB>);
+        &dm::dm_csr_kernel<kOneNS, kOneNG, 3, kOneGroups, kOneMinB>);
     if (!b->one_counts) RBFB_CUDA(ctx, cudaMalloc(&b->one_counts, 3 * kOneKeys * sizeof(int)));
     if (b->one_grid == 0) {
         RBFB_CUDA(ctx, cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, kOneSmem));
@@ -215,7 +214,7 @@ int ensure_one(rbfb_ctx* ctx, BatchState* b) {
         if (nb < 1) return fail(ctx, RBFB_EUNSUPPORTED, "uneven kernel does not fit an SM");
         b->one_grid = nb * ctx->sms;
     }
-    const size_t need = static_cast<size_t>(b->one_grid) * (kOneBlock / 32) * OneCfg::gbytes;
+    const size_t need = static_cast<size_t>(b->one_grid) * kOneGroups * OneCfg::gbytes;
     if (b->gscratch_bytes < need) {
         cudaFree(b->gscratch);
         b->gscratch = nullptr;
@@ -335,7 +334,7 @@ int rbfb_assemble_csr(rbfb_ctx* ctx, const rbfb_desc* desc, int nstencils, const
         q.item_base = 0;
         q.nitems = nstencils;
         q.work = &b->ctrs[0].work[0];
-        blk_csr_kernel<double, kOneNS, kOneNG, 3, kOneBlock, kOnePB, kOneMinB>
+        dm::dm_csr_kernel<kOneNS, kOneNG, 3, kOneGroups, kOneMinB>
             <<<b->one_grid, kOneBlock, kOneSmem, s>>>(q, degree, desc->degree, desc->phs,
                                                        b->gscratch, b->err);
         ctx->launches += 4;

@@ -54,6 +54,7 @@ int rhs_columns(const rbfb_desc* d, AsmParams& p) {
         return RBFB_EINVAL;
     if (m == 0) return RBFB_EINVAL;
     p.nrhs = m;
+    p.plain_ops = (d->ops & ~(RBFB_OP_LAPLACE | RBFB_OP_DX | RBFB_OP_DY)) == 0;
     p.xc = d->xc;
     p.yc = d->yc;
     return m;
