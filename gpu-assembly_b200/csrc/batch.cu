@@ -103,44 +103,84 @@ __global__ void offsets_kernel(int* counts, int nb) {
     }
 }
 
-// Class of every stencil of the single launch (an invalid one gets the
-// last class; the kernel flags it) and the class counts.
-__global__ void one_assign_kernel(int nst, const int* ia, const int8_t* degree, int P0,
-                                  int* key_of, int* counts) {
-    for (int s = blockIdx.x * blockDim.x + threadIdx.x; s < nst; s += gridDim.x * blockDim.x) {
-        const int ks = ia[s + 1] - ia[s];
-        const int P = degree ? degree[s] : P0;
-        int key = kOneKeys - 1;
-        if (P >= 0 && P <= 4 && ks >= 1 && ks + npoly(P) <= kOneNG) key = one_key(ks + npoly(P), P);
-        key_of[s] = key;
-        atomicAdd(counts + key, 1);
-    }
-}
+// Counting sort of the stencils by class for the single launch. A batch has few
+// classes in use, so counters in device memory are contended by every thread
+// (500k stencils: 207 us to count, 249 us to scatter); a block counts in shared
+// memory first and takes one device-wide atomic per class in use.
+constexpr int kSortThreads = 256, kSortPer = 8;  // stencils a thread
 
-__global__ void one_offsets_kernel(int* counts) {
-    __shared__ int part[kOneKeys];
-    for (int i = threadIdx.x; i < kOneKeys; i += blockDim.x) part[i] = counts[i];
+// Class of every stencil (an invalid one gets the last class; the kernel flags
+// it) and the class counts.
+__global__ void __launch_bounds__(kSortThreads)
+    one_assign_kernel(int nst, const int* ia, const int8_t* degree, int P0, int* key_of, int* counts) {
+    __shared__ int h[kOneKeys];
+    for (int i = threadIdx.x; i < kOneKeys; i += kSortThreads) h[i] = 0;
     __syncthreads();
-    if (threadIdx.x == 0) {
-        int acc = 0;
-        for (int i = 0; i < kOneKeys; ++i) {
-            const int c = part[i];
-            part[i] = acc;
-            acc += c;
+    const int s0 = blockIdx.x * (kSortThreads * kSortPer) + threadIdx.x;
+#pragma unroll
+    for (int t = 0; t < kSortPer; ++t) {
+        const int s = s0 + t * kSortThreads;
+        if (s < nst) {
+            const int ks = ia[s + 1] - ia[s];
+            const int P = degree ? degree[s] : P0;
+            int key = kOneKeys - 1;
+            if (P >= 0 && P <= 4 && ks >= 1 && ks + npoly(P) <= kOneNG) key = one_key(ks + npoly(P), P);
+            key_of[s] = key;
+            atomicAdd(h + key, 1);
         }
     }
     __syncthreads();
-    for (int i = threadIdx.x; i < kOneKeys; i += blockDim.x) {
-        counts[kOneKeys + i] = part[i];  // offsets
-        counts[2 * kOneKeys + i] = 0;    // cursors
+    for (int i = threadIdx.x; i < kOneKeys; i += kSortThreads)
+        if (h[i]) atomicAdd(counts + i, h[i]);
+}
+
+// Exclusive scan of the class counts into offsets; cursors to zero. One block
+// of at least kOneKeys threads.
+constexpr int kOneScan = 512;
+static_assert(kOneKeys <= kOneScan, "one thread a class");
+__global__ void __launch_bounds__(kOneScan) one_offsets_kernel(int* counts) {
+    __shared__ int warp_sums[kOneScan / 32];
+    const int i = threadIdx.x, lane = i & 31, w = i >> 5;
+    const int c = i < kOneKeys ? counts[i] : 0;
+    int incl = c;
+    for (int o = 1; o < 32; o <<= 1) {
+        const int t = __shfl_up_sync(0xffffffffu, incl, o);
+        if (lane >= o) incl += t;
+    }
+    if (lane == 31) warp_sums[w] = incl;
+    __syncthreads();
+    int before = 0;
+    for (int v = 0; v < w; ++v) before += warp_sums[v];
+    if (i < kOneKeys) {
+        counts[kOneKeys + i] = before + incl - c;  // offsets
+        counts[2 * kOneKeys + i] = 0;              // cursors
     }
 }
 
-__global__ void one_scatter_kernel(int nst, const int* key_of, int* counts, int* list) {
-    for (int s = blockIdx.x * blockDim.x + threadIdx.x; s < nst; s += gridDim.x * blockDim.x) {
-        const int key = key_of[s];
-        list[counts[kOneKeys + key] + atomicAdd(counts + 2 * kOneKeys + key, 1)] = s;
+__global__ void __launch_bounds__(kSortThreads)
+    one_scatter_kernel(int nst, const int* key_of, int* counts, int* list) {
+    __shared__ int h[kOneKeys];
+    for (int i = threadIdx.x; i < kOneKeys; i += kSortThreads) h[i] = 0;
+    __syncthreads();
+    const int s0 = blockIdx.x * (kSortThreads * kSortPer) + threadIdx.x;
+    const int lane = threadIdx.x & 31;
+    int key[kSortPer], rank[kSortPer];
+#pragma unroll
+    for (int t = 0; t < kSortPer; ++t) {
+        const int s = s0 + t * kSortThreads;
+        key[t] = s < nst ? key_of[s] : -1;
+        const unsigned same = __match_any_sync(0xffffffffu, key[t]);
+        int base = 0;
+        if (key[t] >= 0 && lane == __ffs(same) - 1) base = atomicAdd(h + key[t], __popc(same));
+        rank[t] = __shfl_sync(0xffffffffu, base, __ffs(same) - 1) + __popc(same & ((1u << lane) - 1u));
     }
+    __syncthreads();
+    for (int i = threadIdx.x; i < kOneKeys; i += kSortThreads)
+        if (h[i]) h[i] = counts[kOneKeys + i] + atomicAdd(counts + 2 * kOneKeys + i, h[i]);
+    __syncthreads();
+#pragma unroll
+    for (int t = 0; t < kSortPer; ++t)
+        if (key[t] >= 0) list[h[key[t]] + rank[t]] = s0 + t * kSortThreads;
 }
 
 __global__ void scatter_kernel(int nst, const int* bucket_of, int* counts, int* list) {
@@ -324,11 +364,12 @@ int rbfb_assemble_csr(rbfb_ctx* ctx, const rbfb_desc* desc, int nstencils, const
         if (nstencils == 0) return RBFB_OK;
         // the stencils sorted by class (counting sort on the device)
         RBFB_CUDA(ctx, cudaMemsetAsync(b->one_counts, 0, kOneKeys * sizeof(int), s));
-        const int blocks = std::max(1, std::min((nstencils + 255) / 256, ctx->sms * 8));
-        one_assign_kernel<<<blocks, 256, 0, s>>>(nstencils, ia, degree, desc->degree, b->bucket_of,
-                                                 b->one_counts);
-        one_offsets_kernel<<<1, 256, 0, s>>>(b->one_counts);
-        one_scatter_kernel<<<blocks, 256, 0, s>>>(nstencils, b->bucket_of, b->one_counts, b->list);
+        const int blocks = (nstencils + kSortThreads * kSortPer - 1) / (kSortThreads * kSortPer);
+        one_assign_kernel<<<blocks, kSortThreads, 0, s>>>(nstencils, ia, degree, desc->degree,
+                                                          b->bucket_of, b->one_counts);
+        one_offsets_kernel<<<1, kOneScan, 0, s>>>(b->one_counts);
+        one_scatter_kernel<<<blocks, kSortThreads, 0, s>>>(nstencils, b->bucket_of, b->one_counts,
+                                                           b->list);
         AsmParams q = p;
         q.list = b->list;
         q.item_base = 0;
