@@ -114,6 +114,12 @@ __device__ __forceinline__ void cp_async8(void* dst, const void* src) {
                  "l"(src)
                  : "memory");
 }
+__device__ __forceinline__ void cp_async16(void* dst, const void* src) {
+    asm volatile("cp.async.cg.shared.global [%0], [%1], 16;\n" ::"r"(
+                     (unsigned)__cvta_generic_to_shared(dst)),
+                 "l"(src)
+                 : "memory");
+}
 __device__ __forceinline__ void cp_async_wait_all() { asm volatile("cp.async.wait_all;\n" ::: "memory"); }
 
 // Pivot keys. The magnitude word of a candidate: the bits of |v| for

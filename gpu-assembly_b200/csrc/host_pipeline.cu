@@ -138,9 +138,7 @@ int rbfb_assemble_host(rbfb_ctx* ctx, const rbfb_desc* desc, int n, const double
     } else {
         const double per[2] = {desc->period[0], desc->period[1]};
         const bool periodic = per[0] > 0 && per[1] > 0;
-        rc = knn::build(ctx, n, p->x, p->y, periodic ? per : nullptr, sc);
-        if (rc < 0) return rc;
-        rc = knn::query(ctx, n, nullptr, nullptr, k, p->ja, sc);
+        rc = knn::search(ctx, n, p->x, p->y, 0, nullptr, nullptr, k, periodic ? per : nullptr, p->ja, sc);
         if (rc) return rc;
     }
     if (ja_out_h) {

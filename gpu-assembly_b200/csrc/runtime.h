@@ -100,12 +100,10 @@ int enqueue_fixed(rbfb_ctx* ctx, const rbfb_desc* desc, int first, int count, co
 int check_desc(rbfb_ctx* ctx, const rbfb_desc* d);
 
 namespace knn {
-// Bins the nodes (returns the number of cells or < 0), then answers queries
-// (xq == nullptr: the nodes themselves). Both enqueue on `st`, no sync.
-int build(rbfb_ctx* ctx, int n, const double* x, const double* y, const double* period,
-          cudaStream_t st);
-int query(rbfb_ctx* ctx, int nq, const double* xq, const double* yq, int k, int* ja,
-          cudaStream_t st);
+// The k nearest nodes of every node (xq == nullptr) or of nq query points.
+// Enqueues on `st`, no sync.
+int search(rbfb_ctx* ctx, int n, const double* x, const double* y, int nq, const double* xq,
+           const double* yq, int k, const double* period, int* ja, cudaStream_t st);
 }  // namespace knn
 
 }  // namespace rbfb

@@ -197,8 +197,8 @@ int launch(rbfb_server* s, Slot& sl, Req* r) {
     int rc;
     {
         std::lock_guard<std::mutex> cl(ctx->mu);
-        rc = rbfb::knn::build(ctx, r->n, r->x, r->y, periodic ? per : nullptr, st);
-        if (rc >= 0) rc = rbfb::knn::query(ctx, r->n, nullptr, nullptr, r->k, r->ja, st);
+        rc = rbfb::knn::search(ctx, r->n, r->x, r->y, 0, nullptr, nullptr, r->k,
+                               periodic ? per : nullptr, r->ja, st);
         if (rc >= 0)
             rc = rbfb::enqueue_fixed(ctx, &r->desc, 0, r->n, r->x, r->y, r->k, r->ja, r->vals,
                                      r->info, r->ctr, r->fb, st);
