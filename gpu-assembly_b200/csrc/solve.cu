@@ -58,9 +58,14 @@ constexpr int kChunk = 8;  // iterations between two looks at the stop flag
 // Blocks per SM that stay resident together (at most 40 registers a
 // thread); the grid is that many per SM, so none waits for a second wave.
 constexpr int kBlocksPerSm = 6;
-// The operator passes stage each warp's 32 rows (its entries in one piece,
-// up to kStageEntries) in shared memory: 96 KB a block, two blocks per SM;
-// the same grid then runs in three waves.
+// The vector passes hold four rows' operands in flight: fewer blocks, more
+// registers.
+constexpr int kVectorBlocksPerSm = 4, kUpdateBlocksPerSm = 3;
+// The operator passes stage each warp's rows (its entries in one piece, up to
+// kStageEntries; 32 rows, or 16 at a time) in shared memory: 96 KB a block, two
+// blocks per SM; the same grid then runs in three waves. More blocks with
+// smaller slabs take the L1 that the gathers hit (1M ragged rows, 48
+// iterations: 11.9 ms; three blocks of 768 entries 13.8, four of 576 15.2).
 constexpr int kStageEntries = 1024;
 constexpr int kStagedBlocksPerSm = 2;
 constexpr size_t kStageBytes = static_cast<size_t>(kWarps) * kStageEntries * (sizeof(double) + sizeof(int));
@@ -70,7 +75,7 @@ enum : int { RUNNING = 0, CONVERGED = 1, MAXIT = 2, BREAKDOWN = 3, ZERO_RHS = 4,
 struct State {
     double rho, alpha, omega, beta;
     double ff, thresh2, rr;
-    int iter, maxit, done, pending_breakdown;
+    int iter, maxit, done;
     unsigned int arrive;  // blocks of the running kernel that have finished
     int bad_bnd;          // boundary indices outside [0, n)
 };
@@ -85,7 +90,8 @@ struct Args {
     const double* f;
     double* u;
     double *r, *rh, *p, *v, *s, *t;
-    double* part;  // 3 x gridDim.x partial sums
+    double* part;   // 3 x gridDim.x partial sums of the operator passes
+    double* part2;  // 2 x gridDim.x of the update (and of the initial residual)
     State* st;
 };
 
@@ -146,8 +152,11 @@ __device__ __forceinline__ double row_sum_staged(const double* sval, const int* 
 // copies under an L2 evict-first policy, and each lane sums its own row from
 // there. A piece above kStageEntries (or unaligned arrays) is walked from
 // global memory by row_sum. Same rows, same order, same sums as apply_row.
-template <class W, class F>
-__device__ __forceinline__ void walk_rows(const Args& a, unsigned char* smem, W w, F f) {
+//
+// The first rows' entries are requested before ready() is called: it waits for
+// the kernel's predecessor, and returns false when there is nothing to do.
+template <class R, class W, class F>
+__device__ __forceinline__ bool walk_rows(const Args& a, unsigned char* smem, R ready, W w, F f) {
     const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
     double* sval = reinterpret_cast<double*>(smem) + static_cast<size_t>(wid) * kStageEntries;
     int* sja = reinterpret_cast<int*>(reinterpret_cast<double*>(smem) +
@@ -155,53 +164,65 @@ __device__ __forceinline__ void walk_rows(const Args& a, unsigned char* smem, W 
                static_cast<size_t>(wid) * kStageEntries;
     const unsigned long long pol = evict_first_policy();
     const long long stride = static_cast<long long>(gridDim.x) * kThreads;
+    bool begun = false;
     for (long long t0 = static_cast<long long>(blockIdx.x) * kThreads + wid * 32; t0 < a.n;
          t0 += stride) {
         const long long s = t0 + lane;
-        const long long s1 = min(t0 + 32, static_cast<long long>(a.n));
-        long long q0, q1;
+        const long long sc = min(s, static_cast<long long>(a.n) - 1);
+        long long q, e;
         if (a.ia) {
-            q0 = __ldg(a.ia + t0);
-            q1 = __ldg(a.ia + s1);
+            q = __ldg(a.ia + sc);
+            e = __ldg(a.ia + sc + 1);
         } else {
-            q0 = t0 * a.k;
-            q1 = s1 * a.k;
+            q = sc * a.k;
+            e = q + a.k;
         }
-        const long long qa = q0 & ~3LL;
-        const bool staged = a.vec && q1 - qa <= kStageEntries;
-        if (staged) {
-            const int m = static_cast<int>(q1 - qa);
-            const double* gv = a.values + qa;
-            const int* gj = a.ja + qa;
-            for (int c = lane; c < m / 2; c += 32) cp_async_stream<16>(sval + 2 * c, gv + 2 * c, pol);
-            if ((m & 1) && lane == 0) cp_async_stream<8>(sval + m - 1, gv + m - 1, pol);
-            for (int c = lane; c < m / 4; c += 32) cp_async_stream<16>(sja + 4 * c, gj + 4 * c, pol);
-            for (int e = (m & ~3) + lane; e < m; e += 32) cp_async_stream<4>(sja + e, gj + e, pol);
-            cp_async_commit();
-            cp_async_wait<0>();
-            __syncwarp();
-        }
-        if (s < a.n) {
-            double v;
-            if (a.bflag[s]) {
-                v = w(static_cast<int>(s));
-            } else {
-                long long q, e;
-                if (a.ia) {
-                    q = __ldg(a.ia + s);
-                    e = __ldg(a.ia + s + 1);
-                } else {
-                    q = s * a.k;
-                    e = q + a.k;
-                }
-                v = staged ? row_sum_staged(sval, sja, static_cast<int>(q - qa),
-                                            static_cast<int>(e - qa), w)
-                           : row_sum(a.ja, a.values, q, e, a.vec, w);
+        const bool bnd = a.bflag[sc];
+        for (int r0 = 0, rows = 32; r0 < 32 && t0 + r0 < a.n; r0 += rows) {
+            const long long qa = __shfl_sync(0xffffffffu, q, r0) & ~3LL;
+            long long q1 = __shfl_sync(0xffffffffu, e, r0 + rows - 1);
+            if (rows == 32 && q1 - qa > kStageEntries) {
+                rows = 16;
+                q1 = __shfl_sync(0xffffffffu, e, 15);
             }
-            f(s, v);
+            const bool staged = a.vec && q1 - qa <= kStageEntries;
+            if (staged) {
+                const int m = static_cast<int>(q1 - qa);
+                const double* gv = a.values + qa;
+                const int* gj = a.ja + qa;
+                for (int c = lane; c < m / 2; c += 32)
+                    cp_async_stream<16>(sval + 2 * c, gv + 2 * c, pol);
+                if ((m & 1) && lane == 0) cp_async_stream<8>(sval + m - 1, gv + m - 1, pol);
+                for (int c = lane; c < m / 4; c += 32)
+                    cp_async_stream<16>(sja + 4 * c, gj + 4 * c, pol);
+                for (int i = (m & ~3) + lane; i < m; i += 32) cp_async_stream<4>(sja + i, gj + i, pol);
+                cp_async_commit();
+            }
+            if (!begun) {
+                begun = true;
+                if (!ready()) {
+                    cp_async_wait<0>();
+                    return false;
+                }
+            }
+            if (staged) {
+                cp_async_wait<0>();
+                __syncwarp();
+            }
+            if (lane >= r0 && lane < r0 + rows && s < a.n) {
+                double v;
+                if (bnd)
+                    v = w(static_cast<int>(s));
+                else
+                    v = staged ? row_sum_staged(sval, sja, static_cast<int>(q - qa),
+                                                static_cast<int>(e - qa), w)
+                               : row_sum(a.ja, a.values, q, e, a.vec, w);
+                f(s, v);
+            }
+            __syncwarp();  // the slab is refilled for the next rows
         }
-        __syncwarp();  // the slab is refilled for the next rows
     }
+    return begun || ready();
 }
 
 // Sums NV values over the block; the totals end up in every lane of warp 0.
@@ -226,6 +247,59 @@ __device__ __forceinline__ void block_sum(double (&v)[NV], double (*sh)[NV]) {
     }
 }
 
+// The kernels of an iteration are launched with programmatic stream
+// serialization: a kernel's blocks may start while its predecessor's last ones
+// run. wait_predecessor returns when the predecessor has completed (and with
+// it, since it waited for its own, everything before); start_successor lets the
+// next kernel's blocks start. It comes after the wait, so what a kernel does
+// before its own wait may read anything older than its predecessor.
+__device__ __forceinline__ void wait_predecessor() {
+    asm volatile("griddepcontrol.wait;\n" ::: "memory");
+}
+__device__ __forceinline__ void start_successor() {
+    asm volatile("griddepcontrol.launch_dependents;\n" ::: "memory");
+}
+
+// Waits for the predecessor; false when the solve has stopped.
+__device__ __forceinline__ bool begin_pass(const Args& a) {
+    wait_predecessor();
+    start_successor();
+    return !*reinterpret_cast<volatile int*>(&a.st->done);
+}
+
+// Sums the nb blocks' partial sums of the previous kernel, thread t those of
+// blocks t, t + 256, ..., then the block butterfly: the totals in every thread.
+// Every block of the next kernel does this for itself (at most 21 KB from L2),
+// which costs less than an arrival count and a last block's second pass.
+template <int NV>
+__device__ __forceinline__ void totals(const double* part, int nb, double (&tot)[NV]) {
+    __shared__ double sh[kWarps][NV];
+    __shared__ double res[NV];
+    double g[NV];
+#pragma unroll
+    for (int i = 0; i < NV; ++i) g[i] = 0.0;
+    for (int b = threadIdx.x; b < nb; b += kThreads)
+#pragma unroll
+        for (int i = 0; i < NV; ++i) g[i] += __ldcg(part + i * nb + b);
+    block_sum<NV>(g, sh);
+    if (threadIdx.x == 0)
+#pragma unroll
+        for (int i = 0; i < NV; ++i) res[i] = g[i];
+    __syncthreads();
+#pragma unroll
+    for (int i = 0; i < NV; ++i) tot[i] = res[i];
+}
+
+// The block's partial sums into part.
+template <int NV>
+__device__ __forceinline__ void store_partial(double (&v)[NV], double* part) {
+    __shared__ double sh[kWarps][NV];
+    block_sum<NV>(v, sh);
+    if (threadIdx.x == 0)
+#pragma unroll
+        for (int i = 0; i < NV; ++i) part[i * gridDim.x + blockIdx.x] = v[i];
+}
+
 // Stores the block's partial sums and counts the block in. Returns true in
 // every thread of the block that finished last; tot then holds the grid
 // totals in thread 0 (all of warp 0). The other blocks return false.
@@ -236,7 +310,7 @@ __device__ __forceinline__ bool grid_sum(double (&v)[NV], const Args& a, double 
     block_sum<NV>(v, sh);
     if (threadIdx.x == 0) {
 #pragma unroll
-        for (int i = 0; i < NV; ++i) a.part[i * gridDim.x + blockIdx.x] = v[i];
+        for (int i = 0; i < NV; ++i) a.part2[i * gridDim.x + blockIdx.x] = v[i];
         __threadfence();
         last = atomicAdd(&a.st->arrive, 1u) == gridDim.x - 1;
     }
@@ -248,7 +322,7 @@ __device__ __forceinline__ bool grid_sum(double (&v)[NV], const Args& a, double 
     for (int i = 0; i < NV; ++i) g[i] = 0.0;
     for (int b = threadIdx.x; b < static_cast<int>(gridDim.x); b += kThreads)
 #pragma unroll
-        for (int i = 0; i < NV; ++i) g[i] += __ldcg(a.part + i * gridDim.x + b);
+        for (int i = 0; i < NV; ++i) g[i] += __ldcg(a.part2 + i * gridDim.x + b);
     block_sum<NV>(g, sh);
 #pragma unroll
     for (int i = 0; i < NV; ++i) tot[i] = g[i];
@@ -297,7 +371,6 @@ __global__ void __launch_bounds__(kThreads, kBlocksPerSm) init_kernel(Args a, do
     st->thresh2 = tol * tol * tot[1];
     st->iter = 0;
     st->maxit = maxit;
-    st->pending_breakdown = 0;
     int done = RUNNING;
     if (st->bad_bnd)
         done = BAD_INPUT;  // nothing below may run on an out-of-range boundary list
@@ -313,98 +386,172 @@ __global__ void __launch_bounds__(kThreads, kBlocksPerSm) init_kernel(Args a, do
     st->arrive = 0;
 }
 
-__global__ void __launch_bounds__(kThreads, kBlocksPerSm) p_kernel(Args a) {
-    const State* st = a.st;
-    if (st->done) return;
-    const double beta = st->beta, omega = st->omega;
+// The rows of a vector pass, kUnroll of the thread's (grid-stride) rows at a
+// time: f.load(i, row) for each, then f.store(i, row) in ascending order, so that
+// the loads of kUnroll rows are in flight together.
+constexpr int kUnroll = 4;
+template <class F>
+__device__ __forceinline__ void vector_pass(int n, F& f) {
     const long long stride = static_cast<long long>(gridDim.x) * kThreads;
-    for (long long s = static_cast<long long>(blockIdx.x) * kThreads + threadIdx.x; s < a.n;
-         s += stride)
-        a.p[s] = fma(beta, fma(-omega, a.v[s], a.p[s]), a.r[s]);
+    for (long long s = static_cast<long long>(blockIdx.x) * kThreads + threadIdx.x; s < n;
+         s += kUnroll * stride) {
+#pragma unroll
+        for (int i = 0; i < kUnroll; ++i)
+            if (s + i * stride < n) f.load(i, s + i * stride);
+#pragma unroll
+        for (int i = 0; i < kUnroll; ++i)
+            if (s + i * stride < n) f.store(i, s + i * stride);
+    }
 }
 
-__global__ void __launch_bounds__(kThreads, kStagedBlocksPerSm) spmv_v_kernel(Args a) {
-    State* st = a.st;
+struct PassP {
+    const Args& a;
+    double beta, omega;
+    double v[kUnroll], p[kUnroll], r[kUnroll];
+    __device__ __forceinline__ void load(int i, long long s) {
+        v[i] = a.v[s];
+        p[i] = a.p[s];
+        r[i] = a.r[s];
+    }
+    __device__ __forceinline__ void store(int i, long long s) {
+        a.p[s] = fma(beta, fma(-omega, v[i], p[i]), r[i]);
+    }
+};
+
+__global__ void __launch_bounds__(kThreads, kVectorBlocksPerSm) p_kernel(const __grid_constant__ Args a) {
+    wait_predecessor();
+    start_successor();
+    const State* st = a.st;
     if (st->done) return;
+    PassP f{a, st->beta, st->omega};
+    vector_pass(a.n, f);
+}
+
+__global__ void __launch_bounds__(kThreads, kStagedBlocksPerSm)
+    spmv_v_kernel(const __grid_constant__ Args a) {
     extern __shared__ __align__(16) unsigned char stage_smem[];
     double acc[1] = {0.0};
     const double* p = a.p;
-    walk_rows(a, stage_smem, [p](int j) { return __ldg(p + j); }, [&](long long s, double v) {
-        a.v[s] = v;
-        acc[0] = fma(a.rh[s], v, acc[0]);
-    });
-    double tot[1];
-    if (!grid_sum<1>(acc, a, tot) || threadIdx.x != 0) return;
-    const double sigma = tot[0];
-    if (sigma == 0.0 || !is_fin(sigma))
-        st->done = BREAKDOWN;
-    else
-        st->alpha = st->rho / sigma;
-    st->arrive = 0;
+    const bool run = walk_rows(
+        a, stage_smem, [&] { return begin_pass(a); }, [p](int j) { return p[j]; },
+        [&](long long s, double v) {
+            a.v[s] = v;
+            acc[0] = fma(a.rh[s], v, acc[0]);
+        });
+    if (!run) return;
+    store_partial<1>(acc, a.part);
 }
 
-__global__ void __launch_bounds__(kThreads, kBlocksPerSm) s_kernel(Args a) {
-    const State* st = a.st;
-    if (st->done) return;
-    const double alpha = st->alpha;
-    const long long stride = static_cast<long long>(gridDim.x) * kThreads;
-    for (long long i = static_cast<long long>(blockIdx.x) * kThreads + threadIdx.x; i < a.n;
-         i += stride)
-        a.s[i] = fma(-alpha, a.v[i], a.r[i]);
-}
+struct PassS {
+    const Args& a;
+    double alpha;
+    double v[kUnroll], r[kUnroll];
+    __device__ __forceinline__ void load(int i, long long s) {
+        v[i] = a.v[s];
+        r[i] = a.r[s];
+    }
+    __device__ __forceinline__ void store(int i, long long s) { a.s[s] = fma(-alpha, v[i], r[i]); }
+};
 
-__global__ void __launch_bounds__(kThreads, kStagedBlocksPerSm) spmv_t_kernel(Args a) {
+// sigma = (rh, v), alpha = rho / sigma, then s = r - alpha v. Every block forms
+// alpha; the first one stores it.
+__global__ void __launch_bounds__(kThreads, kVectorBlocksPerSm) s_kernel(const __grid_constant__ Args a) {
+    wait_predecessor();
+    start_successor();
     State* st = a.st;
-    if (st->done) return;
+    // one read of the flag a block: the first block may set it below, and then
+    // every block finds the same breakdown
+    __shared__ int done;
+    if (threadIdx.x == 0) done = *reinterpret_cast<volatile int*>(&st->done);
+    __syncthreads();
+    if (done) return;
+    double tot[1];
+    totals<1>(a.part, gridDim.x, tot);
+    const double sigma = tot[0];
+    const bool broken = sigma == 0.0 || !is_fin(sigma);
+    const double alpha = broken ? 0.0 : st->rho / sigma;
+    if (blockIdx.x == 0 && threadIdx.x == 0) {
+        if (broken)
+            st->done = BREAKDOWN;
+        else
+            st->alpha = alpha;
+    }
+    if (broken) return;
+    PassS f{a, alpha};
+    vector_pass(a.n, f);
+}
+
+__global__ void __launch_bounds__(kThreads, kStagedBlocksPerSm)
+    spmv_t_kernel(const __grid_constant__ Args a) {
     extern __shared__ __align__(16) unsigned char stage_smem[];
     double acc[3] = {0.0, 0.0, 0.0};
     const double* sv = a.s;
-    walk_rows(a, stage_smem, [sv](int j) { return __ldg(sv + j); }, [&](long long i, double ti) {
-        const double si = sv[i];
-        a.t[i] = ti;
-        acc[0] = fma(ti, si, acc[0]);
-        acc[1] = fma(ti, ti, acc[1]);
-        acc[2] = fma(si, si, acc[2]);
-    });
-    double tot[3];
-    if (!grid_sum<3>(acc, a, tot) || threadIdx.x != 0) return;
-    if (tot[2] <= st->thresh2) {
-        st->omega = 0.0;  // s is small enough: u += alpha p finishes the solve
-    } else if (tot[1] == 0.0 || !is_fin(tot[1]) || !is_fin(tot[0])) {
-        st->omega = 0.0;
-        st->pending_breakdown = 1;
-    } else {
-        st->omega = tot[0] / tot[1];
-    }
-    st->arrive = 0;
+    const bool run = walk_rows(
+        a, stage_smem, [&] { return begin_pass(a); }, [sv](int j) { return sv[j]; },
+        [&](long long i, double ti) {
+            const double si = sv[i];
+            a.t[i] = ti;
+            acc[0] = fma(ti, si, acc[0]);
+            acc[1] = fma(ti, ti, acc[1]);
+            acc[2] = fma(si, si, acc[2]);
+        });
+    if (!run) return;
+    store_partial<3>(acc, a.part);
 }
 
-__global__ void __launch_bounds__(kThreads, kBlocksPerSm) update_kernel(Args a) {
+struct PassUpdate {
+    const Args& a;
+    double alpha, omega;
+    double acc0, acc1;
+    double si[kUnroll], p[kUnroll], u[kUnroll], t[kUnroll], rh[kUnroll];
+    __device__ __forceinline__ void load(int i, long long s) {
+        si[i] = a.s[s];
+        p[i] = a.p[s];
+        u[i] = a.u[s];
+        t[i] = a.t[s];
+        rh[i] = a.rh[s];
+    }
+    __device__ __forceinline__ void store(int i, long long s) {
+        a.u[s] = fma(omega, si[i], fma(alpha, p[i], u[i]));
+        const double ri = fma(-omega, t[i], si[i]);
+        a.r[s] = ri;
+        acc0 = fma(rh[i], ri, acc0);
+        acc1 = fma(ri, ri, acc1);
+    }
+};
+
+// omega from (t, s), (t, t), (s, s), then u and r, and the last block the next
+// iteration's coefficients and the stop flag.
+__global__ void __launch_bounds__(kThreads, kUpdateBlocksPerSm)
+    update_kernel(const __grid_constant__ Args a) {
+    wait_predecessor();
+    start_successor();
     State* st = a.st;
     if (st->done) return;
-    const double alpha = st->alpha, omega = st->omega;
-    double acc[2] = {0.0, 0.0};
-    const long long stride = static_cast<long long>(gridDim.x) * kThreads;
-    for (long long i = static_cast<long long>(blockIdx.x) * kThreads + threadIdx.x; i < a.n;
-         i += stride) {
-        const double si = a.s[i];
-        a.u[i] = fma(omega, si, fma(alpha, a.p[i], a.u[i]));
-        const double ri = fma(-omega, a.t[i], si);
-        a.r[i] = ri;
-        acc[0] = fma(a.rh[i], ri, acc[0]);
-        acc[1] = fma(ri, ri, acc[1]);
+    double tot3[3];
+    totals<3>(a.part, gridDim.x, tot3);
+    double omega = 0.0;  // s small enough: u += alpha p finishes the solve
+    bool broken = false;
+    if (!(tot3[2] <= st->thresh2)) {
+        broken = tot3[1] == 0.0 || !is_fin(tot3[1]) || !is_fin(tot3[0]);
+        if (!broken) omega = tot3[0] / tot3[1];
     }
+    const double alpha = st->alpha;
+    PassUpdate f{a, alpha, omega, 0.0, 0.0};
+    vector_pass(a.n, f);
+    double acc[2] = {f.acc0, f.acc1};
     double tot[2];
     if (!grid_sum<2>(acc, a, tot) || threadIdx.x != 0) return;
     const double rho_new = tot[0], rr = tot[1];
     st->iter += 1;
     st->rr = rr;
+    st->omega = omega;
     int done = RUNNING;
     if (!is_fin(rr))
         done = BREAKDOWN;
     else if (rr <= st->thresh2)
         done = CONVERGED;
-    else if (st->pending_breakdown || omega == 0.0)
+    else if (broken || omega == 0.0)
         done = BREAKDOWN;
     else if (st->iter >= st->maxit)
         done = MAXIT;
@@ -468,7 +615,7 @@ int ensure(rbfb_ctx* ctx, int n, int grid) {
         if (w->part) cudaFree(w->part);
         w->part = nullptr;
         w->grid_cap = 0;
-        if (cudaMalloc(&w->part, 3 * sizeof(double) * grid) != cudaSuccess) {
+        if (cudaMalloc(&w->part, 5 * sizeof(double) * grid) != cudaSuccess) {
             cudaGetLastError();
             return fail(ctx, RBFB_ENOMEM, "solve workspace");
         }
@@ -477,18 +624,32 @@ int ensure(rbfb_ctx* ctx, int n, int grid) {
     return RBFB_OK;
 }
 
+// One kernel of an iteration, allowed to start while its predecessor ends.
+cudaError_t launch(void (*kern)(Args), int grid, size_t smem, cudaStream_t st, const Args& a) {
+    cudaLaunchAttribute attr{};
+    attr.id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    attr.val.programmaticStreamSerializationAllowed = 1;
+    cudaLaunchConfig_t c{};
+    c.gridDim = dim3(grid);
+    c.blockDim = dim3(kThreads);
+    c.dynamicSmemBytes = smem;
+    c.stream = st;
+    c.attrs = &attr;
+    c.numAttrs = 1;
+    return cudaLaunchKernelEx(&c, kern, a);
+}
+
 // Enqueues kChunk iterations (5 launches each).
 int enqueue_chunk(rbfb_ctx* ctx, const Args& a, int grid, cudaStream_t st) {
     for (int it = 0; it < kChunk; ++it) {
-        p_kernel<<<grid, kThreads, 0, st>>>(a);
-        spmv_v_kernel<<<grid, kThreads, kStageBytes, st>>>(a);
-        s_kernel<<<grid, kThreads, 0, st>>>(a);
-        spmv_t_kernel<<<grid, kThreads, kStageBytes, st>>>(a);
-        update_kernel<<<grid, kThreads, 0, st>>>(a);
+        RBFB_CUDA(ctx, launch(p_kernel, grid, 0, st, a));
+        RBFB_CUDA(ctx, launch(spmv_v_kernel, grid, kStageBytes, st, a));
+        RBFB_CUDA(ctx, launch(s_kernel, grid, 0, st, a));
+        RBFB_CUDA(ctx, launch(spmv_t_kernel, grid, kStageBytes, st, a));
+        RBFB_CUDA(ctx, launch(update_kernel, grid, 0, st, a));
         ctx->launches += 5;
     }
-    const cudaError_t e = cudaGetLastError();
-    return e == cudaSuccess ? RBFB_OK : cuda_fail(ctx, e, "solve kernels");
+    return RBFB_OK;
 }
 
 }  // namespace solve
@@ -539,6 +700,7 @@ extern "C" int rbfb_solve_bicgstab(rbfb_ctx* ctx, int n, int k, const int* ia, c
     a.s = vec + 4 * static_cast<size_t>(n);
     a.t = vec + 5 * static_cast<size_t>(n);
     a.part = w->part;
+    a.part2 = w->part + 3 * static_cast<size_t>(grid);
     a.st = w->st;
 
     RBFB_CUDA(ctx, cudaMemsetAsync(w->st, 0, sizeof(State), st));
