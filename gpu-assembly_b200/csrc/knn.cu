@@ -237,6 +237,116 @@ __global__ void scatter_kernel(const double* x, const double* y, int n, const Gr
     }
 }
 
+// All of the binning in one block, for small node sets, whose search would
+// otherwise be mostly launches: 4,761 nodes in the open plane, k = 21, binning
+// and query 41 us in seven launches, 28 in two (with the smaller cells of per_cell).
+// One block is bound by its chain of barriers and memory latencies, ~12 us, which
+// grows with n: at 8,192 nodes 33 us against 41 (periodic 35 against 38), and
+// more nodes a thread would not fit its registers.
+// Each thread keeps its nodes in registers; the cell counts and their scan live
+// in shared memory.
+constexpr int kSmallNodes = 8192, kSmallPer = kSmallNodes / 1024;
+constexpr int kSmallCells = kSmallNodes / kPerCell, kSmallCellsPer = kSmallCells / 1024;
+__global__ void __launch_bounds__(1024) small_bins_kernel(const double* x, const double* y, int n, int cells,
+                                                          double per, Grid gv, Grid* gp, Head* head,
+                                                          int* start, int* rank, int* sidx,
+                                                          double2* sxy) {
+    __shared__ int count[kSmallCells];
+    __shared__ double sh[32][4];
+    __shared__ int warp_sums[32];
+    __shared__ Grid g;
+    const int tid = threadIdx.x, lane = tid & 31, w = tid >> 5;
+    double px[kSmallPer], py[kSmallPer];
+#pragma unroll
+    for (int j = 0; j < kSmallPer; ++j) {
+        const int i = tid + 1024 * j;
+        px[j] = i < n ? x[i] : 0.0;
+        py[j] = i < n ? y[i] : 0.0;
+    }
+#pragma unroll
+    for (int j = 0; j < kSmallCellsPer; ++j) count[tid + 1024 * j] = 0;
+    if (gp) {
+        double m[4] = {-1e308, -1e308, -1e308, -1e308};
+#pragma unroll
+        for (int j = 0; j < kSmallPer; ++j)
+            if (tid + 1024 * j < n) {
+                m[0] = fmax(m[0], -px[j]);
+                m[1] = fmax(m[1], px[j]);
+                m[2] = fmax(m[2], -py[j]);
+                m[3] = fmax(m[3], py[j]);
+            }
+#pragma unroll
+        for (int j = 0; j < 4; ++j) {
+            for (int o = 16; o > 0; o >>= 1) m[j] = fmax(m[j], __shfl_xor_sync(0xffffffffu, m[j], o));
+            if (lane == 0) sh[w][j] = m[j];
+        }
+        __syncthreads();
+        if (w == 0) {
+#pragma unroll
+            for (int j = 0; j < 4; ++j) {
+                m[j] = sh[lane][j];
+                for (int o = 16; o > 0; o >>= 1)
+                    m[j] = fmax(m[j], __shfl_xor_sync(0xffffffffu, m[j], o));
+            }
+            if (lane == 0) g = open_grid(-m[0], m[1], -m[2], m[3], cells, per);
+        }
+    } else if (tid == 0) {
+        g = gv;
+    }
+    __syncthreads();
+    if (tid == 0) {
+        head->status = 0;
+        if (gp) *gp = g;
+    }
+    int cell[kSmallPer], rk[kSmallPer];
+#pragma unroll
+    for (int j = 0; j < kSmallPer; ++j) {
+        if (tid + 1024 * j < n) {
+            px[j] = fold(px[j], g.Lx);
+            py[j] = fold(py[j], g.Ly);
+            cell[j] = cell_coord(py[j], g.y0, g.hy, g.cy) * g.cx + cell_coord(px[j], g.x0, g.hx, g.cx);
+            rk[j] = atomicAdd(count + cell[j], 1);
+        }
+    }
+    __syncthreads();
+    // exclusive scan, kSmallCellsPer consecutive cells a thread
+    int v[kSmallCellsPer], own = 0;
+#pragma unroll
+    for (int j = 0; j < kSmallCellsPer; ++j) {
+        v[j] = count[tid * kSmallCellsPer + j];
+        own += v[j];
+    }
+    int incl = own;
+    for (int o = 1; o < 32; o <<= 1) {
+        const int t = __shfl_up_sync(0xffffffffu, incl, o);
+        if (lane >= o) incl += t;
+    }
+    if (lane == 31) warp_sums[w] = incl;
+    __syncthreads();
+    int before = lane < w ? warp_sums[lane] : 0;
+    for (int o = 16; o > 0; o >>= 1) before += __shfl_xor_sync(0xffffffffu, before, o);
+    int at = before + incl - own;
+#pragma unroll
+    for (int j = 0; j < kSmallCellsPer; ++j) {
+        const int c = tid * kSmallCellsPer + j;
+        count[c] = at;
+        if (c <= cells) start[c] = at;
+        at += v[j];
+    }
+    if (tid == 1023 && cells == kSmallCells) start[cells] = at;
+    __syncthreads();
+#pragma unroll
+    for (int j = 0; j < kSmallPer; ++j) {
+        const int i = tid + 1024 * j;
+        if (i < n) {
+            const int pos = count[cell[j]] + rk[j];
+            rank[i] = 0;  // no mark of the general search (cell_query_kernel)
+            sidx[pos] = i;
+            sxy[pos] = make_double2(px[j], py[j]);
+        }
+    }
+}
+
 // ---- 3. queries --------------------------------------------------------------------
 struct QueryArgs {
     const Grid* g;     // device grid, or nullptr: gv
@@ -871,10 +981,14 @@ int ensure_ws(rbfb_ctx* ctx, size_t n, size_t cells) {
 // more queries. Measured for (k + 4 sqrt k) / 12.6, 10, 8, 7 nodes a cell: 631,
 // 614, 728, 537 us (1M disk, k = 21), 891, 911, 951, 973 (1M periodic, k =
 // 35), 1542, 773, 732, 676 (300k nodes of fourfold varying density, k = 64).
+// A small set takes smaller cells, down to what two rings need for k, so that
+// there is a cell for every resident warp (4,761 nodes, k = 21: query 18 -> 12 us).
 // Arbitrary query points: kPerCell.
-double per_cell(int k, bool own) {
-    return own ? std::max<double>(kPerCell, (k + 4.0 * std::sqrt(static_cast<double>(k))) / 7.0)
-               : kPerCell;
+double per_cell(int k, int n, int sms, bool own) {
+    if (!own) return kPerCell;
+    const double root = std::sqrt(static_cast<double>(k));
+    const double least = (k + 1 + 2.0 * root) / 11.4, most = (k + 4.0 * root) / 7.0;
+    return std::max<double>(kPerCell, std::min(most, std::max(least, n / (16.0 * sms))));
 }
 
 // The cell grid over n nodes: its cells (periodic: its geometry too; open
@@ -889,11 +1003,19 @@ size_t plan_grid(int n, const double* period, double per, Grid& g) {
     return static_cast<size_t>(cx) * cy;
 }
 
-// Enqueues the binning of the nodes into the arrays of w (five launches and a
-// memset, six in the open plane); gp: the device grid (open plane) or nullptr
-// (periodic: gv). Returns the first error.
+// Enqueues the binning of the nodes into the arrays of w (one launch for a small
+// set, else a memset and four launches, five in the open plane, one fewer when
+// one block scans all cells); gp: the device grid (open plane) or nullptr
+// (periodic: gv); *launches is increased. Returns the first error.
 cudaError_t enqueue_bins(const Workspace& w, int n, const double* x, const double* y, size_t cells,
-                         double per, const Grid* gp, const Grid& gv, int sms, cudaStream_t st) {
+                         double per, const Grid* gp, const Grid& gv, int sms, cudaStream_t st,
+                         int* launches) {
+    if (n <= kSmallNodes && cells <= kSmallCells) {
+        small_bins_kernel<<<1, 1024, 0, st>>>(x, y, n, static_cast<int>(cells), per, gv, gp ? w.grid : nullptr,
+                                              w.head, w.start, w.rank, w.sidx, w.sxy);
+        *launches += 1;
+        return cudaGetLastError();
+    }
     const int ncell1 = static_cast<int>(cells) + 1;
     int* count = reinterpret_cast<int*>(w.head + 1);
     const cudaError_t e = cudaMemsetAsync(w.head, 0, sizeof(Head) + ncell1 * sizeof(int), st);
@@ -908,6 +1030,7 @@ cudaError_t enqueue_bins(const Workspace& w, int n, const double* x, const doubl
     scan_block_kernel<<<nsb, kScanBlock, 0, st>>>(count, w.start, ncell1, w.block_sums);
     if (nsb > 1) scan_add_kernel<<<nsb, kScanBlock, 0, st>>>(w.start, ncell1, w.block_sums);
     scatter_kernel<<<blocks, tpb, 0, st>>>(x, y, n, gp, gv, w.cell_of, w.rank, w.start, w.sidx, w.sxy);
+    *launches += 3 + (gp ? 1 : 0) + (nsb > 1 ? 1 : 0);
     return cudaGetLastError();
 }
 
@@ -957,15 +1080,16 @@ bool is_periodic(const double* period) { return period && period[0] > 0 && perio
 int search(rbfb_ctx* ctx, int n, const double* x, const double* y, int nq, const double* xq,
            const double* yq, int k, const double* period, int* ja, cudaStream_t st) {
     const bool periodic = is_periodic(period);
-    const double per = per_cell(k, !xq);
+    const double per = per_cell(k, n, ctx->sms, !xq);
     Grid gv{};
     const size_t cells = plan_grid(n, periodic ? period : nullptr, per, gv);
     const int rc = ensure_ws(ctx, n, cells);
     if (rc) return rc;
     const Workspace& w = *ws_of(ctx);
     const Grid* gp = periodic ? nullptr : w.grid;
-    RBFB_CUDA(ctx, enqueue_bins(w, n, x, y, cells, per, gp, gv, ctx->sms, st));
-    ctx->launches += periodic ? 4 : 5;
+    int launches = 0;
+    RBFB_CUDA(ctx, enqueue_bins(w, n, x, y, cells, per, gp, gv, ctx->sms, st, &launches));
+    ctx->launches += launches;
     QueryArgs a = query_args(w, gp, gv, k, ja);
     if (!xq) {
         RBFB_CUDA(ctx, enqueue_cells(a, cells, periodic, ctx->sms, st));
@@ -1112,13 +1236,16 @@ extern "C" int rbfb_knn_stencils_static(int n, const double* x, const double* y,
     if (period_h && ((period_h[0] > 0) != (period_h[1] > 0))) return RBFB_EINVAL;
     if (n > kStaticMaxNodes) return RBFB_ETOOBIG;
     // the cell grid of the search, as rbfb_knn_stencils forms it
-    const double per = per_cell(k, true);
-    Grid gv{};
-    const size_t cells = plan_grid(n, periodic ? period_h : nullptr, per, gv);
-    if (cells > static_cast<size_t>(kStaticMaxCells)) return RBFB_ETOOBIG;
     int dev = 0;
     unsigned char* base = static_scratch(&dev);
     if (!base) return RBFB_ECUDA;
+    int sms = 0;
+    cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
+    sms = std::max(sms, 1);
+    const double per = per_cell(k, n, sms, true);
+    Grid gv{};
+    const size_t cells = plan_grid(n, periodic ? period_h : nullptr, per, gv);
+    if (cells > static_cast<size_t>(kStaticMaxCells)) return RBFB_ETOOBIG;
     Workspace w;
     w.cell_of = reinterpret_cast<int*>(base + kS_cell_of);
     w.rank = reinterpret_cast<int*>(base + kS_rank);
@@ -1129,11 +1256,9 @@ extern "C" int rbfb_knn_stencils_static(int n, const double* x, const double* y,
     w.sxy = reinterpret_cast<double2*>(base + kS_sxy);
     w.grid = reinterpret_cast<Grid*>(base + kS_grid);
     cudaStream_t st = static_cast<cudaStream_t>(stream);
-    int sms = 0;
-    cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
-    sms = std::max(sms, 1);
     const Grid* gp = periodic ? nullptr : w.grid;
-    if (enqueue_bins(w, n, x, y, cells, per, gp, gv, sms, st) != cudaSuccess ||
+    int launches = 0;
+    if (enqueue_bins(w, n, x, y, cells, per, gp, gv, sms, st, &launches) != cudaSuccess ||
         enqueue_cells(query_args(w, gp, gv, k, ja), cells, periodic, sms, st) != cudaSuccess)
         return RBFB_ECUDA;
     return RBFB_OK;

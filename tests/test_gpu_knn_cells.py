@@ -101,3 +101,12 @@ def test_variable_density(ctx, torch_cuda, k):
     _check(ctx, torch_cuda, x, y, k)
     x, y, _ = NS.unit_disk(4000, nb=200, seed=k)
     _check(ctx, torch_cuda, x, y, k)
+
+
+# the largest set that one block bins, and the smallest that the grid does
+@pytest.mark.parametrize("n", [8192, 8193])
+@pytest.mark.parametrize("make", [_clusters, _coincident, _line, _channel, _lattice])
+def test_either_side_of_the_one_block_binning(ctx, torch_cuda, make, n):
+    x, y = make(np.random.default_rng(n), n)
+    for k, period in ((21, None), (35, (2.0, 3.0))):
+        _check(ctx, torch_cuda, x, y, k, period)
