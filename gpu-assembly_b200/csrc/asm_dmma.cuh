@@ -53,7 +53,7 @@
 
 #include <cstdint>
 
-#include "asm_kernel.cuh"
+#include "asm_common.cuh"
 
 namespace rbfb {
 namespace dm {
@@ -546,7 +546,7 @@ __device__ __forceinline__ void panel_careful(double* S, const uint8_t* list, ui
         const uint32_t best = __reduce_max_sync(ALL, key);
         if (best < 128u && info == 0) info = c0 + t + 1;  // zero pivot column
         const int pos = 127 - (int)(best & 127u);
-        const double rv = recip_rn(bv);
+        const double rv = __drcp_rn(bv);
         const double inv = __shfl_sync(ALL, rv, pos & 31);
 #pragma unroll
         for (int sl = 0; sl < R; ++sl) {

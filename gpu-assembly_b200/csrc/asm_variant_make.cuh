@@ -4,56 +4,31 @@
 
 #include <cuda_runtime.h>
 
-#include "asm_blocked.cuh"
 #include "asm_dmma.cuh"
-#include "asm_kernel.cuh"
+#include "asm_common.cuh"
+#include "asm_refined.cuh"
 #include "asm_variants.h"
 
 namespace rbfb {
 
-template <typename T, int GR, int GC, int NTP, int NRHS, int P, int Q, bool MIXED, int BLOCK,
-          int MINB, bool SMEM, bool PF>
-Variant make_variant(const char* name) {
-    using C = AsmCfg<T, GR, GC, NTP, NRHS, P, Q, MIXED, SMEM>;
+template <int NMAX, int NRHS, int P, int Q, int GPB, int MINB>
+Variant make_ir_variant(const char* name) {
+    using L = ir::Layout<NMAX, NRHS, NMAX - npoly(P)>;
     Variant v{};
     v.name = name;
-    v.kernel =
-        reinterpret_cast<const void*>(&asm_kernel<T, GR, GC, NTP, NRHS, P, Q, MIXED, BLOCK, MINB, SMEM, PF>);
+    v.kernel = reinterpret_cast<const void*>(&ir::ir_kernel<NMAX, NRHS, P, Q, GPB, MINB>);
     v.launch = [](dim3 grid, int block, size_t smem, cudaStream_t st, const AsmParams& p) {
-        asm_kernel<T, GR, GC, NTP, NRHS, P, Q, MIXED, BLOCK, MINB, SMEM, PF><<<grid, block, smem, st>>>(p);
+        ir::ir_kernel<NMAX, NRHS, P, Q, GPB, MINB><<<grid, block, smem, st>>>(p);
     };
-    v.mixed = MIXED;
-    v.P = P;
-    v.Q = Q;
-    v.ntp = NTP;
-    v.nrhs = NRHS;
-    v.group = C::G;
-    v.block = BLOCK;
-    v.smem_group = C::bytes;
-    v.smem_block = C::bytes * (BLOCK / C::G);
-    return v;
-}
-
-template <typename T, int NMAX, int NRHS, int P, int Q, bool MIXED, int BLOCK, int MINB, int PB,
-          bool PF>
-Variant make_blk_variant(const char* name) {
-    using C = BlkCfg<T, NMAX, NRHS, P, Q, MIXED, PB>;
-    Variant v{};
-    v.name = name;
-    v.kernel = reinterpret_cast<const void*>(
-        &blk_kernel<T, NMAX, NRHS, P, Q, MIXED, BLOCK, MINB, PB, PF>);
-    v.launch = [](dim3 grid, int block, size_t smem, cudaStream_t st, const AsmParams& p) {
-        blk_kernel<T, NMAX, NRHS, P, Q, MIXED, BLOCK, MINB, PB, PF><<<grid, block, smem, st>>>(p);
-    };
-    v.mixed = MIXED;
+    v.mixed = true;
     v.P = P;
     v.Q = Q;
     v.ntp = NMAX;
     v.nrhs = NRHS;
-    v.group = C::G;
-    v.block = BLOCK;
-    v.smem_group = C::bytes;
-    v.smem_block = C::bytes * (BLOCK / C::G);
+    v.group = 32;
+    v.block = 32 * GPB;
+    v.smem_group = L::bytes;
+    v.smem_block = L::bytes * GPB;
     return v;
 }
 
@@ -87,16 +62,7 @@ Variant make_dm_variant(const char* name) {
     }                                                                                          \
     }
 
-#define RBFB_DEFINE_BLK_VARIANT(name, T, NMAX, NRHS, P, Q, MIXED, BLOCK, MINB, PB, PF)          \
+#define RBFB_DEFINE_IR_VARIANT(name, NMAX, NRHS, P, Q, GPB, MINB)                               \
     namespace rbfb {                                                                           \
-    Variant variant_##name() {                                                                 \
-        return make_blk_variant<T, NMAX, NRHS, P, Q, MIXED, BLOCK, MINB, PB, PF>(#name);       \
-    }                                                                                          \
-    }
-
-#define RBFB_DEFINE_VARIANT(name, T, GR, GC, NTP, NRHS, P, Q, MIXED, BLOCK, MINB, SMEM, PF)    \
-    namespace rbfb {                                                                           \
-    Variant variant_##name() {                                                                 \
-        return make_variant<T, GR, GC, NTP, NRHS, P, Q, MIXED, BLOCK, MINB, SMEM, PF>(#name);  \
-    }                                                                                          \
+    Variant variant_##name() { return make_ir_variant<NMAX, NRHS, P, Q, GPB, MINB>(#name); }   \
     }

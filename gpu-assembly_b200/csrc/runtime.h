@@ -12,7 +12,7 @@
 #include <vector>
 
 #include "rbf_b200.h"
-#include "asm_kernel.cuh"
+#include "asm_common.cuh"
 #include "asm_variants.h"
 
 namespace rbfb {
