@@ -28,6 +28,7 @@
 #include <cstdint>
 
 #include "rbf_b200.h"
+#include "row_sum.cuh"
 #include "stream_copy.cuh"
 
 namespace rbfb {
@@ -190,41 +191,44 @@ __global__ void bgk_kernel(int n, T omega, T* __restrict__ pdf, T* __restrict__ 
 
 constexpr int kTileWarps = 4;  // warps a CTA; each warp owns a 32-node tile at a time
 
-// Shared memory of one warp: DEPTH weight slabs (the directions in flight)
-// and the tile's index slab, 32 rows of ks entries each; ks = k for odd k,
-// k + 1 for even k, so that row r of lane r is bank-conflict free.
-inline int tile_stride(int k) { return (k & 1) ? k : k + 1; }
-inline size_t tile_smem_bytes(int k, int depth, bool jreg) {
-    return static_cast<size_t>(kTileWarps) * 32 * tile_stride(k) *
-           (depth * sizeof(double) + (jreg ? 0 : sizeof(int)));
+// How a tile's rows are copied into its slabs: in 16-byte pieces of one run, in
+// 16-byte pieces row by row (k a multiple of 4: rows one after another would put
+// all lanes on a few banks), or entry by entry (arrays that are not 16-byte
+// aligned; an even k is padded to the next odd).
+enum Copy { kRun16, kRows16, kRun8, kPad8 };
+
+// Entries from a row to the next in shared memory.
+template <int COPY>
+__host__ __device__ constexpr int weight_stride(int k) {
+    return COPY == kRows16 ? k + 2 : COPY == kPad8 ? k + 1 : k;
+}
+template <int COPY>
+__host__ __device__ inline int index_stride(int k) {
+    return COPY == kRows16 ? (k / 4 % 2 ? k : k + 4) : COPY == kPad8 ? k + 1 : k;
 }
 
-// Copies the tile's m = cnt * k consecutive entries (element e to row e / k,
-// column e % k of a ks-strided slab); lane takes e = lane + 32 i. (r, c) is
-// the row and column of the lane's current element, advanced by 32 entries.
-// VEC (unpadded slabs, 16-byte aligned source and destination): 16-byte
-// copies, the odd tail entries one by one.
-template <bool PAD, bool VEC, typename V>
+// Copies the tile's m entries of rows of k into a slab of stride ks.
+template <int COPY, typename V>
 __device__ __forceinline__ void copy_slab(V* dst, const V* src, int m, int k, int ks, int lane,
-                                          int r, int c, int q32, int r32,
                                           unsigned long long pol) {
-    if constexpr (VEC && !PAD) {
-        constexpr int per = 16 / sizeof(V);
+    constexpr int per = 16 / sizeof(V);
+    if constexpr (COPY == kRun16) {
         const int chunks = m / per;
         for (int q = lane; q < chunks; q += 32)
             cp_async_stream<16>(dst + q * per, src + q * per, pol);
         for (int e = chunks * per + lane; e < m; e += 32)
             cp_async_stream<sizeof(V)>(dst + e, src + e, pol);
     } else {
-        for (int e = lane; e < m; e += 32) {
-            cp_async_stream<sizeof(V)>(dst + (PAD ? r * ks + c : e), src + e, pol);
-            if (PAD) {
-                r += q32;
-                c += r32;
-                if (c >= k) {
-                    c -= k;
-                    ++r;
-                }
+        constexpr int step = COPY == kRows16 ? per : 1;
+        const int row = k / step, q32 = 32 / row, r32 = 32 - q32 * row;
+        int r = lane / row, c = lane - r * row;  // of this lane's piece
+        for (int q = lane; q < m / step; q += 32) {
+            cp_async_stream<step * sizeof(V)>(dst + r * ks + c * step, src + q * step, pol);
+            r += q32;
+            c += r32;
+            if (c >= row) {
+                c -= row;
+                ++r;
             }
         }
     }
@@ -234,93 +238,92 @@ __device__ __forceinline__ void copy_slab(V* dst, const V* src, int m, int k, in
 // interpolation operators W (8 arrays of n*k weights, direction a at
 // W + (a-1)*n*k, rows like ja), then the BGK collision, into pdf_out. The
 // moments of the streamed populations go to rho, ux, uy (any may be null).
-// A warp takes a tile of 32 consecutive nodes: it copies the tile's index
-// rows and the first DEPTH - 1 directions' weight rows into shared memory;
-// for each direction it starts the copy of the direction DEPTH - 1 ahead and
-// has each lane sum its own node's row in entry order (the first product
-// rounded, then one fused multiply-add an entry), gathering pdf_in through
-// the indices. Then every lane collides its node and the warp writes 32
-// consecutive entries of each direction, as streaming stores. KT > 0 fixes
-// k at compile time (the row's gathers all in flight at once). JREG (with
-// KT): the index rows land in the second weight buffer and each lane keeps
-// its own row in registers for the tile, so no index slab is kept.
-template <typename T, bool PAD, int KT, int DEPTH, bool VEC, bool JREG = false>
-__global__ void __launch_bounds__(kTileWarps * 32) stream_collide_kernel(
+// A warp takes a tile of 32 consecutive nodes: it copies the tile's index rows
+// and the first direction's weight rows into shared memory; for each direction
+// it starts the copy of the next one and has each lane sum its own node's row in
+// entry order (the first product rounded, then one fused multiply-add an entry),
+// gathering pdf_in through the indices. Then every lane collides its node and the
+// warp writes 32 consecutive entries of each direction, as streaming stores.
+//
+// Bound by memory where enough warps are resident to cover the gathers, so:
+// KT > 0 fixes k at compile time: the index rows land in the second weight slab
+// and each lane keeps its own in registers for the tile, which saves the index
+// slab and its reads, and the gathers of a row are in flight at once.
+// 1M nodes (100k), FP64, us: k = 15 264 -> 188 (42 -> 22), k = 18 361 -> 218 (47
+// -> 27), k = 21 265 -> 248 (37 -> 31), k = 24 589 -> 312 (64 -> 38); 6.4 TB/s at
+// k = 21. Before, even k was copied entry by entry and the sizes other than 21 read
+// their indices from a slab for every direction.
+// Resident CTAs that the registers are cut for: those that the slabs allow, at
+// most 6 for short rows and 4 (128 registers) from 16 entries on, where more
+// gathers in flight are worth more than more warps. 1M nodes, k = 15 187 (6) and
+// 195 us (4), k = 16 223 and 209, k = 21 254 and 248; left to itself the compiler
+// takes 56 registers for k = 21 in FP32, 330 us against 229.
+constexpr int resident(int kt, int stride) {
+    const int fit = 227 * 1024 / (kTileWarps * 32 * 2 * stride * 8 + 1024);
+    const int most = kt > 0 && kt < 16 ? 6 : 4;
+    return kt == 0 ? most : fit < most ? fit : most;
+}
+template <typename T, int COPY, int KT>
+__global__ void __launch_bounds__(kTileWarps * 32, resident(KT, weight_stride<COPY>(KT)))
+    stream_collide_kernel(
     int n, int k, const int* __restrict__ ja, const double* __restrict__ W, T omega,
     const T* __restrict__ pdf_in, T* __restrict__ pdf_out, T* __restrict__ rho,
     T* __restrict__ ux, T* __restrict__ uy) {
-    static_assert(DEPTH >= 2 && DEPTH <= 4, "prefetch depth");
-    static_assert(!JREG || (KT > 0 && !PAD && DEPTH == 2), "index rows in registers");
     extern __shared__ __align__(16) unsigned char tile_smem[];
     if (KT > 0) k = KT;
     const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
-    const int ks = PAD ? k + 1 : k;
-    const int slab = 32 * ks;
-    double* wbuf =
-        reinterpret_cast<double*>(tile_smem) + static_cast<size_t>(wid) * DEPTH * slab;
-    int* jbuf = JREG ? reinterpret_cast<int*>(wbuf + slab)
-                     : reinterpret_cast<int*>(reinterpret_cast<double*>(tile_smem) +
-                                              static_cast<size_t>(kTileWarps) * DEPTH * slab) +
-                           static_cast<size_t>(wid) * slab;
+    const int kv = weight_stride<COPY>(k), kj = index_stride<COPY>(k);
+    const int slab = 32 * kv;
+    double* wbuf = reinterpret_cast<double*>(tile_smem) + static_cast<size_t>(wid) * 2 * slab;
+    int* jbuf = KT ? reinterpret_cast<int*>(wbuf + slab)
+                   : reinterpret_cast<int*>(reinterpret_cast<double*>(tile_smem) +
+                                            static_cast<size_t>(kTileWarps) * 2 * slab) +
+                         static_cast<size_t>(wid) * 32 * kj;
     const size_t N = static_cast<size_t>(n);
     const size_t nnz = N * static_cast<size_t>(k);
     const unsigned long long pol = evict_first_policy();
-    const int r0 = lane / k, c0 = lane - r0 * k, q32 = 32 / k, r32 = 32 - q32 * k;
     const int tiles = (n + 31) >> 5;
     for (int tile = blockIdx.x * kTileWarps + wid; tile < tiles; tile += gridDim.x * kTileWarps) {
         const int s0 = tile << 5;
         const int cnt = min(32, n - s0);
         const int m = cnt * k;
         const size_t base = static_cast<size_t>(s0) * k;
-        copy_slab<PAD, VEC>(jbuf, ja + base, m, k, ks, lane, r0, c0, q32, r32, pol);
-#pragma unroll
-        for (int d = 1; d < DEPTH; ++d) {
-            copy_slab<PAD, VEC>(wbuf + (d - 1) * slab, W + static_cast<size_t>(d - 1) * nnz + base,
-                                m, k, ks, lane, r0, c0, q32, r32, pol);
-            cp_async_commit();
-        }
-        int jrow[JREG ? KT : 1];
-        if constexpr (JREG) {  // the lane's index row, then the buffer is free
+        copy_slab<COPY>(jbuf, ja + base, m, k, kj, lane, pol);
+        copy_slab<COPY>(wbuf, W + base, m, k, kv, lane, pol);
+        cp_async_commit();
+        int jrow[KT ? KT : 1];
+        if constexpr (KT > 0) {  // the lane's index row, then the slab is free
             cp_async_wait<0>();
             __syncwarp();
             if (lane < cnt)
 #pragma unroll
-                for (int j = 0; j < KT; ++j) jrow[j] = jbuf[lane * ks + j];
+                for (int j = 0; j < KT; ++j) jrow[j] = jbuf[lane * kj + j];
             __syncwarp();
         }
         T f[9];
 #pragma unroll
         for (int a = 1; a < 9; ++a) {
-            const int nxt = a + DEPTH - 1;  // the direction whose copy starts now
-            if (nxt <= 8) {
-                copy_slab<PAD, VEC>(wbuf + ((nxt - 1) % DEPTH) * slab,
-                                    W + static_cast<size_t>(nxt - 1) * nnz + base, m, k, ks, lane,
-                                    r0, c0, q32, r32, pol);
+            if (a < 8) {
+                copy_slab<COPY>(wbuf + (a & 1) * slab, W + static_cast<size_t>(a) * nnz + base, m, k, kv,
+                                lane, pol);
                 cp_async_commit();
             }
-            cp_async_wait_pending(min(DEPTH - 1, 8 - a));
+            cp_async_wait_pending(a < 8 ? 1 : 0);
             __syncwarp();
             if (lane < cnt) {
-                const double* wr = wbuf + ((a - 1) % DEPTH) * slab + lane * ks;
-                const int* jr = jbuf + lane * ks;
+                const double* wr = wbuf + ((a - 1) & 1) * slab + lane * kv;
                 const T* pa = pdf_in + N * a;
-                T v;
-                if constexpr (JREG) {
-                    v = mul(static_cast<T>(wr[0]), pa[jrow[0]]);
+                if constexpr (KT > 0) {
+                    T v = mul(static_cast<T>(wr[0]), pa[jrow[0]]);
 #pragma unroll
                     for (int j = 1; j < KT; ++j) v = fmaT(static_cast<T>(wr[j]), pa[jrow[j]], v);
-                } else if constexpr (KT > 0) {
-                    v = mul(static_cast<T>(wr[0]), pa[jr[0]]);
-#pragma unroll
-                    for (int j = 1; j < KT; ++j) v = fmaT(static_cast<T>(wr[j]), pa[jr[j]], v);
+                    f[a] = v;
                 } else {
-                    v = mul(static_cast<T>(wr[0]), pa[jr[0]]);
-#pragma unroll 8
-                    for (int j = 1; j < k; ++j) v = fmaT(static_cast<T>(wr[j]), pa[jr[j]], v);
+                    // a sum from -0 gives the first product itself
+                    f[a] = row_sum_shared<8>(wr, jbuf + lane * kj, k, [pa](int c) { return pa[c]; }, T(-0.0));
                 }
-                f[a] = v;
             }
-            __syncwarp();  // every lane is done with this buffer before it is refilled
+            __syncwarp();  // every lane is done with this slab before it is refilled
         }
         const int s = s0 + lane;
         if (lane < cnt) {
@@ -336,11 +339,13 @@ __global__ void __launch_bounds__(kTileWarps * 32) stream_collide_kernel(
     }
 }
 
-template <typename T, bool PAD, int KT, int DEPTH, bool VEC, bool JREG = false>
+template <typename T, int COPY, int KT>
 int launch_stream_collide(int n, int k, const int* ja, const double* W, T omega, const T* pin,
                           T* pout, T* rho, T* ux, T* uy, cudaStream_t st) {
-    auto kern = stream_collide_kernel<T, PAD, KT, DEPTH, VEC, JREG>;
-    const size_t smem = tile_smem_bytes(k, DEPTH, JREG);
+    auto kern = stream_collide_kernel<T, COPY, KT>;
+    const size_t smem = static_cast<size_t>(kTileWarps) * 32 *
+                        (2 * weight_stride<COPY>(k) * sizeof(double) +
+                         (KT ? 0 : index_stride<COPY>(k) * sizeof(int)));
     if (cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize,
                              static_cast<int>(smem)) != cudaSuccess)
         return RBFB_ECUDA;
@@ -358,26 +363,33 @@ int launch_stream_collide(int n, int k, const int* ja, const double* W, T omega,
     return cudaGetLastError() == cudaSuccess ? RBFB_OK : RBFB_ECUDA;
 }
 
+// A kernel for each stencil size up to kMaxFixed, from kMinFixed (degree 1) on.
+constexpr int kMinFixed = 5, kMaxFixed = 32;
+template <typename T, int KT, class... A>
+int launch_fixed(int n, int k, A... args) {
+    if constexpr (KT > kMaxFixed) {
+        return launch_stream_collide<T, kRun16, 0>(n, k, args...);
+    } else {
+        if (k != KT) return launch_fixed<T, KT + 1>(n, k, args...);
+        return launch_stream_collide<T, KT % 4 ? kRun16 : kRows16, KT>(n, k, args...);
+    }
+}
+
 template <typename T>
 int stream_collide(int n, int k, const int* ja, const double* W, T omega, const T* pin, T* pout,
                    T* rho, T* ux, T* uy, cudaStream_t st) {
     // 16-byte copies need 16-byte aligned rows: ja, W and every direction's
-    // array (n*k even). Odd k: unpadded slabs; k = 21 (the D2Q9 operators'
-    // usual stencil) fixed at compile time, with the index rows held in
-    // registers. Even k: padded slabs, 8-byte copies.
+    // array (n*k even)
     const bool vec = ((reinterpret_cast<uintptr_t>(ja) | reinterpret_cast<uintptr_t>(W)) & 15) == 0 &&
                      ((static_cast<long long>(n) * k) & 1) == 0;
-    if (!(k & 1))
-        return launch_stream_collide<T, true, 0, 2, false>(n, k, ja, W, omega, pin, pout, rho, ux,
-                                                           uy, st);
-    if (vec && k == 21)  // index rows in registers: no index slab, 20 warps per SM
-        return launch_stream_collide<T, false, 21, 2, true, true>(n, k, ja, W, omega, pin, pout,
-                                                                  rho, ux, uy, st);
-    if (vec)
-        return launch_stream_collide<T, false, 0, 2, true>(n, k, ja, W, omega, pin, pout, rho, ux,
-                                                           uy, st);
-    return launch_stream_collide<T, false, 0, 2, false>(n, k, ja, W, omega, pin, pout, rho, ux,
-                                                        uy, st);
+    if (vec && k >= kMinFixed && k <= kMaxFixed)
+        return launch_fixed<T, kMinFixed>(n, k, ja, W, omega, pin, pout, rho, ux, uy, st);
+    if (vec && k % 4 == 0)
+        return launch_stream_collide<T, kRows16, 0>(n, k, ja, W, omega, pin, pout, rho, ux, uy, st);
+    if (vec) return launch_stream_collide<T, kRun16, 0>(n, k, ja, W, omega, pin, pout, rho, ux, uy, st);
+    if (k & 1)
+        return launch_stream_collide<T, kRun8, 0>(n, k, ja, W, omega, pin, pout, rho, ux, uy, st);
+    return launch_stream_collide<T, kPad8, 0>(n, k, ja, W, omega, pin, pout, rho, ux, uy, st);
 }
 
 int blocks_for(int n) {

@@ -61,4 +61,32 @@ __device__ __forceinline__ double row_sum(const int* __restrict__ ja,
     return acc;
 }
 
+__device__ __forceinline__ double fused(double a, double b, double c) { return __fma_rn(a, b, c); }
+__device__ __forceinline__ float fused(float a, float b, float c) { return __fmaf_rn(a, b, c); }
+
+// The same sum over a row staged in shared memory, m entries (v, j), from acc:
+// B gathers in flight, the last batch's too.
+template <int B, class T, class X>
+__device__ __forceinline__ T row_sum_shared(const double* v, const int* j, int m, X x, T acc) {
+    int i = 0;
+#pragma unroll 1
+    for (; i + B <= m; i += B) {
+        T w[B];
+#pragma unroll
+        for (int c = 0; c < B; ++c) w[c] = x(j[i + c]);
+#pragma unroll
+        for (int c = 0; c < B; ++c) acc = fused(static_cast<T>(v[i + c]), w[c], acc);
+    }
+    if (i < m) {
+        T w[B - 1];
+#pragma unroll
+        for (int c = 0; c < B - 1; ++c)
+            if (i + c < m) w[c] = x(j[i + c]);
+#pragma unroll
+        for (int c = 0; c < B - 1; ++c)
+            if (i + c < m) acc = fused(static_cast<T>(v[i + c]), w[c], acc);
+    }
+    return acc;
+}
+
 }  // namespace rbfb

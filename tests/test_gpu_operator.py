@@ -68,3 +68,42 @@ def test_solve_row_lengths(ctx, torch_cuda, k, n, ragged):
                                     tol=1e-12, maxit=400, grid=O.solve_grid(n, sms))
     assert it == oit and rel == orel and (st == R.OK) == (ost == 0)
     np.testing.assert_array_equal(u.cpu().numpy(), ou)
+
+
+# operators past L2: blocks of four warps
+@pytest.mark.parametrize("n,k", [(700003, 17), (500001, 24), (330000, 35)])
+def test_spmv_large(torch_cuda, n, k):
+    T = torch_cuda
+    rng = np.random.default_rng(k)
+    ja = rng.integers(0, n, (n, k), dtype=np.int32).ravel()
+    v, u = rng.standard_normal(n * k), rng.standard_normal(n)
+    bnd = np.arange(0, n, 1000, dtype=np.int32)
+    jd, vd, ud, bd = (T.as_tensor(a).cuda() for a in (ja, v, u, bnd))
+    out = T.empty(n, dtype=T.float64, device="cuda")
+    R.spmv(n, k, jd, vd, ud, out, bd)
+    np.testing.assert_array_equal(out.cpu().numpy(), O.spmv(ja, v, u, k, bnd))
+
+
+# the streaming step at every stencil size: a kernel each up to 32 entries, the
+# general one past them; whole and ragged tiles; arrays that are not 16-byte
+# aligned
+@pytest.mark.parametrize("dtype", [np.float64, np.float32])
+@pytest.mark.parametrize("k", list(range(1, 41)) + [48, 63, 64])
+def test_stream_collide_every_row_length(torch_cuda, dtype, k):
+    T = torch_cuda
+    rng = np.random.default_rng(k)
+    for n, shift in ((64, 0), (301, 0), (302, 0), (302, 1)):
+        ja = rng.integers(0, n, n * k, dtype=np.int32)
+        W = rng.standard_normal(8 * n * k)
+        W[rng.random(W.size) < 0.1] = -0.0
+        f = rng.uniform(0.5, 1.5, 9 * n).astype(dtype)
+        store = T.zeros(8 * n * k + shift, dtype=T.float64, device="cuda")
+        Wd = store[shift:]
+        Wd.copy_(T.as_tensor(W))
+        jd, fd = T.as_tensor(ja).cuda(), T.as_tensor(f).cuda()
+        out = T.full((9 * n,), 7.0, dtype=fd.dtype, device="cuda")
+        m = [T.empty(n, dtype=fd.dtype, device="cuda") for _ in range(3)]
+        R.lbm_stream_collide(k, jd, Wd, 1.2, fd, out, *m)
+        want = O.lbm_stream_collide(k, ja, W, 1.2, f)
+        for got, w in zip([out] + m, want):
+            np.testing.assert_array_equal(got.cpu().numpy(), w)
