@@ -124,33 +124,13 @@ __device__ __forceinline__ double apply_row(const Args& a, long long s, W w) {
     return row_sum(a.ja, a.values, q, e, a.vec, w);
 }
 
-// Row sum over staged entries lo .. hi-1 of the warp's slab, in row order
-// (the sums of row_sum), eight gathers of w in flight (sixteen measured
-// slower).
-template <class W>
-__device__ __forceinline__ double row_sum_staged(const double* sval, const int* sja, int lo,
-                                                 int hi, W w) {
-    double acc = 0.0;
-    int q = lo;
-    for (; q + 8 <= hi; q += 8) {
-        double v[8], x[8];
-#pragma unroll
-        for (int i = 0; i < 8; ++i) x[i] = w(sja[q + i]);
-#pragma unroll
-        for (int i = 0; i < 8; ++i) v[i] = sval[q + i];
-#pragma unroll
-        for (int i = 0; i < 8; ++i) acc = fma(v[i], x[i], acc);
-    }
-    for (; q < hi; ++q) acc = fma(sval[q], w(sja[q]), acc);
-    return acc;
-}
-
 // This thread's rows in ascending order (the grid-stride rows of apply_row's
 // callers), each as f(s, (A w)_s). A warp takes its 32 consecutive rows at
 // once: their entries (one contiguous piece of ja and values, from a 4-entry
 // boundary) are copied into the warp's shared-memory slab with 16-byte
 // copies under an L2 evict-first policy, and each lane sums its own row from
-// there. A piece above kStageEntries (or unaligned arrays) is walked from
+// there (eight gathers of w in flight; sixteen measured
+// slower). A piece above kStageEntries (or unaligned arrays) is walked from
 // global memory by row_sum. Same rows, same order, same sums as apply_row.
 //
 // The first rows' entries are requested before ready() is called: it waits for
@@ -214,8 +194,7 @@ __device__ __forceinline__ bool walk_rows(const Args& a, unsigned char* smem, R 
                 if (bnd)
                     v = w(static_cast<int>(s));
                 else
-                    v = staged ? row_sum_staged(sval, sja, static_cast<int>(q - qa),
-                                                static_cast<int>(e - qa), w)
+                    v = staged ? row_sum_shared<8>(sval + (q - qa), sja + (q - qa), static_cast<int>(e - q), w, 0.0)
                                : row_sum(a.ja, a.values, q, e, a.vec, w);
                 f(s, v);
             }

@@ -24,22 +24,24 @@ namespace rbfb {
 // line per lane and load: 1.6 GB through the L1s for 437 MB of operator, and the
 // L1 bound it. 16 rows a warp leave room for 32 warps per SM. 1M rows, k = 35:
 // 128 -> 79 us (5.5 TB/s of the operator's bytes); 32 rows a warp, 16 warps: 92.
-// k a multiple of 4 would put the rows of all lanes on a few banks: they are
-// copied one by one with padding (PAD).
+// k a multiple of 4 would put the rows of all lanes on a few banks: their rows
+// are padded by a 16-byte piece (PAD; 60,000 rows, k = 36: 9.9 us, 10.0 walked).
 constexpr int kSpmvWarps = 4, kTileRows = 16;
 struct TileShape {
     int rows;    // rows a warp
     int kv, kj;  // entries from a row to the next in shared memory: weights, columns
+    int mv, mj;  // padded rows: 2^16 / (16-byte pieces a row), rounded up
     __host__ __device__ size_t warp_bytes() const {
         return (static_cast<size_t>(rows) * kv + 4) / 2 * 16 + (static_cast<size_t>(rows) * kj + 7) / 4 * 16;
     }
 };
 inline TileShape tile_shape(int k) {
-    // 48 entries a row, padded: 8 rows 31.6 us (150k rows), 16 33.6
-    TileShape t{k <= 17 ? 32 : k % 4 == 0 && k >= 44 ? 8 : kTileRows, k, k};
+    TileShape t{k <= 17 ? 32 : kTileRows, k, k, 0, 0};
     if (k % 4 == 0) {
         t.kv = k + 2;
         t.kj = k / 4 % 2 ? k : k + 4;
+        t.mv = (65536 + k / 2 - 1) / (k / 2);
+        t.mj = (65536 + k / 4 - 1) / (k / 4);
     }
     return t;
 }
@@ -55,24 +57,20 @@ __global__ void __launch_bounds__(kSpmvWarps * 32, 8)
     int* sj = reinterpret_cast<int*>(sv + (t.rows * t.kv + 4) / 2 * 2);
     const unsigned long long pol = evict_first_policy();
     const int tiles = (n + t.rows - 1) / t.rows;
-    // PAD: this lane's first 16-byte chunk of weights and of columns, and the step
-    // of 32 chunks, as (row, chunk in the row)
-    const int cv = k / 2, cj = k / 4;
-    for (int tile = blockIdx.x * kSpmvWarps + wid; tile < tiles; tile += gridDim.x * kSpmvWarps) {
+    const int warps = blockDim.x >> 5;
+    for (int tile = blockIdx.x * warps + wid; tile < tiles; tile += gridDim.x * warps) {
         const int s0 = tile * t.rows, rows = min(t.rows, n - s0);
         const long long q0 = static_cast<long long>(s0) * k, qa = PAD ? q0 : q0 & ~3LL;
         const int m = static_cast<int>(q0 - qa) + rows * k;
         const double* gv = values + qa;
         const int* gj = ja + qa;
         if constexpr (PAD) {
-            for (int c = lane, r = lane / cv, i = lane - r * cv; c < m / 2; c += 32) {
-                cp_async_stream<16>(sv + r * t.kv + 2 * i, gv + 2 * c, pol);
-                for (i += 32; i >= cv; i -= cv) ++r;
-            }
-            for (int c = lane, r = lane / cj, i = lane - r * cj; c < m / 4; c += 32) {
-                cp_async_stream<16>(sj + r * t.kj + 4 * i, gj + 4 * c, pol);
-                for (i += 32; i >= cj; i -= cj) ++r;
-            }
+            // the row of piece c, c / (pieces a row), by a product: exact for every
+            // tile (at most 1,024 pieces)
+            for (int c = lane; c < m / 2; c += 32)
+                cp_async_stream<16>(sv + 2 * c + ((c * t.mv) >> 16) * (t.kv - k), gv + 2 * c, pol);
+            for (int c = lane; c < m / 4; c += 32)
+                cp_async_stream<16>(sj + 4 * c + ((c * t.mj) >> 16) * (t.kj - k), gj + 4 * c, pol);
         } else {
             for (int c = lane; c < m / 2; c += 32) cp_async_stream<16>(sv + 2 * c, gv + 2 * c, pol);
             if ((m & 1) && lane == 0) cp_async_stream<8>(sv + m - 1, gv + m - 1, pol);
@@ -86,18 +84,7 @@ __global__ void __launch_bounds__(kSpmvWarps * 32, 8)
             const int lead = static_cast<int>(q0 - qa);
             const double* v = sv + lead + lane * t.kv;
             const int* j = sj + lead + lane * t.kj;
-            double acc = 0.0;
-            int i = 0;
-#pragma unroll 1
-            for (; i + 8 <= k; i += 8) {
-                double x[8];
-#pragma unroll
-                for (int c = 0; c < 8; ++c) x[c] = __ldg(u + j[i + c]);
-#pragma unroll
-                for (int c = 0; c < 8; ++c) acc = fma(v[i + c], x[c], acc);
-            }
-            for (; i < k; ++i) acc = fma(v[i], __ldg(u + j[i]), acc);
-            out[s0 + lane] = acc;
+            out[s0 + lane] = row_sum_shared<8>(v, j, k, [u](int c) { return __ldg(u + c); }, 0.0);
         }
         __syncwarp();  // the slab is refilled
     }
@@ -114,6 +101,7 @@ __global__ void spmv_fixed_kernel(int n, int k, const int* __restrict__ ja,
 }
 
 constexpr int kTiledMaxK = 128;  // above: the slabs leave too few warps
+constexpr long long kL2Bytes = 126ll * 1000 * 1000;
 
 int launch_spmv(int n, int k, const int* ja, const double* values, const double* u, double* out,
                 cudaStream_t st) {
@@ -124,14 +112,19 @@ int launch_spmv(int n, int k, const int* ja, const double* values, const double*
         return RBFB_OK;
     }
     const TileShape t = tile_shape(k);
-    const size_t smem = kSpmvWarps * t.warp_bytes();
+    // Blocks of one warp even out the last wave, which counts while the operator
+    // comes from L2 (k = 35, 150,000 rows: 15.2 us, four warps 17.9); beyond it, and
+    // for the few warps that long rows leave, four are as good or better (k = 44,
+    // 700,000 rows: 80 against 84; k = 60, 60,000 rows: 14.5 against 15.9).
+    const int warps = k < 60 && static_cast<long long>(n) * k * 12 <= kL2Bytes ? 1 : kSpmvWarps;
+    const size_t smem = warps * t.warp_bytes();
     auto* kern = k % 4 == 0 ? &spmv_tiled_kernel<true> : &spmv_tiled_kernel<false>;
     if (smem > 48 * 1024 && cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                                  static_cast<int>(smem)) != cudaSuccess)
         return RBFB_ECUDA;
-    const int per_block = kSpmvWarps * t.rows;
-    const int blocks = std::min((n + per_block - 1) / per_block, 148 * 64);
-    kern<<<blocks, kSpmvWarps * 32, smem, st>>>(n, k, t, ja, values, u, out);
+    const int per_block = warps * t.rows;
+    const int blocks = std::min((n + per_block - 1) / per_block, 148 * 256 / warps);
+    kern<<<blocks, warps * 32, smem, st>>>(n, k, t, ja, values, u, out);
     return RBFB_OK;
 }
 
