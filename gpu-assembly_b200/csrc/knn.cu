@@ -16,9 +16,9 @@
 //      when at least k are, the k nearest are among them. They are ranked by a
 //      counting sort on the squared distance (uniform over the circle, so the
 //      buckets hold about half an entry) and exact comparisons inside a
-//      bucket. Queries it cannot complete, and arbitrary query points
-//      (query_kernel), take the general search: one warp per query, a block
-//      that grows until k are found, ranking by comparison.
+//      bucket. Queries it cannot complete (leftover_kernel) and arbitrary
+//      query points (query_kernel) take the general search: one warp per query,
+//      a block that grows until k are found, ranking by comparison.
 //
 // Distances use the reference's arithmetic exactly: dx*dx + dy*dy of the
 // plain differences, each operation rounded (nanoflann L2_Simple_Adaptor,
@@ -60,7 +60,8 @@ struct Head {
     unsigned long long bbox[4];  // ordered images: max of -x, x, -y, y
     unsigned int ticket;         // blocks of the bounding-box kernel that are done
     int status;                  // 1: a query could not be completed
-    int pad[6];
+    int left;                    // queries that the search by cells left over
+    int pad[5];
 };
 static_assert(sizeof(Head) == 64, "the counts after it stay aligned");
 
@@ -249,7 +250,7 @@ constexpr int kSmallNodes = 8192, kSmallPer = kSmallNodes / 1024;
 constexpr int kSmallCells = kSmallNodes / kPerCell, kSmallCellsPer = kSmallCells / 1024;
 __global__ void __launch_bounds__(1024) small_bins_kernel(const double* x, const double* y, int n, int cells,
                                                           double per, Grid gv, Grid* gp, Head* head,
-                                                          int* start, int* rank, int* sidx,
+                                                          int* start, int* sidx,
                                                           double2* sxy) {
     __shared__ int count[kSmallCells];
     __shared__ double sh[32][4];
@@ -296,6 +297,7 @@ __global__ void __launch_bounds__(1024) small_bins_kernel(const double* x, const
     __syncthreads();
     if (tid == 0) {
         head->status = 0;
+        head->left = 0;
         if (gp) *gp = g;
     }
     int cell[kSmallPer], rk[kSmallPer];
@@ -340,7 +342,6 @@ __global__ void __launch_bounds__(1024) small_bins_kernel(const double* x, const
         const int i = tid + 1024 * j;
         if (i < n) {
             const int pos = count[cell[j]] + rk[j];
-            rank[i] = 0;  // no mark of the general search (cell_query_kernel)
             sidx[pos] = i;
             sxy[pos] = make_double2(px[j], py[j]);
         }
@@ -360,10 +361,12 @@ struct QueryArgs {
     int k;
     int* ja;
     int* status;  // set to 1 when a query could not be completed
-    // cell_query_kernel: capacities of a warp's shared-memory lists; marks (< 0)
-    // of the nodes, in cell order, that are left to the general search
+    // cell_query_kernel: capacities of a warp's shared-memory lists; the nodes
+    // (in cell order) that it leaves to leftover_kernel and their number
     int cand_cap, keep_cap;
-    int* undone;
+    int split;  // warps a cell
+    int* list;
+    int* left;
 };
 
 __device__ __forceinline__ bool key_less(unsigned long long da, int ia, unsigned long long db,
@@ -632,25 +635,32 @@ __global__ void __launch_bounds__(kWarps * 32, 8) query_kernel(QueryArgs a) {
         search_one(a, g, fold(a.qx[q], g.Lx), fold(a.qy[q], g.Ly), q, sd[w], si[w], lane);
 }
 
-// The general search of node t (in cell order), out of line.
-__device__ __noinline__ void search_node(const QueryArgs& a, int t, unsigned char* scratch, int lane) {
+// The nodes that the search by cells left over, one warp each (the warp of
+// their cell would take them one after another: 11,359 nodes of fourfold varying
+// density, k = 61: 261 -> 141 us; 60,000 of a disk 331 -> 252). The launch costs a
+// set that leaves none 2 us.
+__global__ void __launch_bounds__(kWarps * 32, 8) leftover_kernel(QueryArgs a) {
+    __shared__ unsigned long long sd[kWarps][kCap];
+    __shared__ int si[kWarps][kCap];
+    const int w = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    const int count = *a.left;
+    if (count == 0) return;
     const Grid g = a.g ? *a.g : a.gv;
-    const double2 q = a.sxy[t];
-    search_one(a, g, q.x, q.y, a.sidx[t], reinterpret_cast<unsigned long long*>(scratch),
-               reinterpret_cast<int*>(scratch + kCap * 8), lane);
+    for (int i = blockIdx.x * kWarps + w; i < count; i += gridDim.x * kWarps) {
+        const int t = a.list[i];
+        const double2 q = a.sxy[t];
+        search_one(a, g, q.x, q.y, a.sidx[t], sd[w], si[w], lane);
+    }
 }
 
 // ---- the nodes' own stencils, cell by cell ------------------------------------
 constexpr int kBuckets = 128;  // of the counting sort: four a lane
 
 // Shared memory of one warp: the block's candidates (coordinates, node
-// indices), the kept ones (distance, node index) and the buckets. The general
-// search reuses it.
+// indices), the kept ones (distance, node index) and the buckets.
 __host__ __device__ constexpr size_t cell_smem(int cand_cap, int keep_cap) {
-    const size_t b = static_cast<size_t>(cand_cap) * 20 + static_cast<size_t>(keep_cap) * 12 +
-                     (kBuckets + 4) * 4;
-    const size_t least = kCap * 12;
-    return ((b > least ? b : least) + 15) & ~size_t(15);
+    return (static_cast<size_t>(cand_cap) * 20 + static_cast<size_t>(keep_cap) * 12 +
+            (kBuckets + 4) * 4 + 15) & ~size_t(15);
 }
 
 // Ranks the `have` kept entries (kd: bits of the squared distance, ki: node
@@ -743,11 +753,13 @@ __global__ void __launch_bounds__(kWarps * 32, NSMAX > 5 ? 6 : 8) cell_query_ker
     __shared__ Grid g;
     if (threadIdx.x == 0) g = a.g ? *a.g : a.gv;
     __syncthreads();
-    const int k = a.k, ncells = g.cx * g.cy;
+    const int k = a.k, items = g.cx * g.cy * a.split;
     const float want = (k + 1 + 1.9f * sqrtf(k + 1.0f)) / 3.14159265f;
-    bool again = false;
-    for (int cell = blockIdx.x * kWarps + w; cell < ncells; cell += gridDim.x * kWarps) {
-        const int q0 = a.start[cell], q1 = a.start[cell + 1];
+    for (int item = blockIdx.x * kWarps + w; item < items; item += gridDim.x * kWarps) {
+        // this warp's part of the cell's nodes
+        const int cell = item / a.split, part = item - cell * a.split;
+        const int first = a.start[cell], own = a.start[cell + 1] - first;
+        const int q0 = first + own * part / a.split, q1 = first + own * (part + 1) / a.split;
         if (q0 == q1) continue;
         const int ccy = cell / g.cx, ccx = cell - ccy * g.cx;
         for (int qb = q0; qb < q1; qb += 32) {
@@ -910,22 +922,14 @@ __global__ void __launch_bounds__(kWarps * 32, NSMAX > 5 ? 6 : 8) cell_query_ker
                 pending = failed;
                 ++R;
             }
-            // what neither block completed waits for the general search below (its
-            // call, in here, would cost the loop its registers)
-            if (pending) {
-                if ((pending >> lane) & 1u) a.undone[qb + lane] = -1;
-                again = true;
+            if (pending) {  // what neither block completed
+                int at = 0;
+                if (lane == 0) at = atomicAdd(a.left, __popc(pending));
+                at = __shfl_sync(0xffffffffu, at, 0);
+                if ((pending >> lane) & 1u) a.list[at + __popc(pending & ((1u << lane) - 1u))] = qb + lane;
             }
         }
     }
-    if (!again) return;
-    for (int cell = blockIdx.x * kWarps + w; cell < ncells; cell += gridDim.x * kWarps)
-        for (int t = a.start[cell]; t < a.start[cell + 1]; ++t)
-            if (a.undone[t] < 0) {
-                __syncwarp();
-                search_node(a, t, base, lane);
-                __syncwarp();
-            }
 }
 
 struct Workspace {
@@ -981,13 +985,14 @@ int ensure_ws(rbfb_ctx* ctx, size_t n, size_t cells) {
 // more queries. Measured for (k + 4 sqrt k) / 12.6, 10, 8, 7 nodes a cell: 631,
 // 614, 728, 537 us (1M disk, k = 21), 891, 911, 951, 973 (1M periodic, k =
 // 35), 1542, 773, 732, 676 (300k nodes of fourfold varying density, k = 64).
-// A small set takes smaller cells, down to what two rings need for k, so that
-// there is a cell for every resident warp (4,761 nodes, k = 21: query 18 -> 12 us).
+// A small set takes smaller cells, towards a cell for every resident warp, down to
+// 1.3 times what two rings need for k (1.0 times leaves many nodes of a varying
+// density over: 11,359 nodes, k = 61, 226 us against 106).
 // Arbitrary query points: kPerCell.
 double per_cell(int k, int n, int sms, bool own) {
     if (!own) return kPerCell;
     const double root = std::sqrt(static_cast<double>(k));
-    const double least = (k + 1 + 2.0 * root) / 11.4, most = (k + 4.0 * root) / 7.0;
+    const double least = (k + 1 + 2.0 * root) / 8.8, most = (k + 4.0 * root) / 7.0;
     return std::max<double>(kPerCell, std::min(most, std::max(least, n / (16.0 * sms))));
 }
 
@@ -1012,7 +1017,7 @@ cudaError_t enqueue_bins(const Workspace& w, int n, const double* x, const doubl
                          int* launches) {
     if (n <= kSmallNodes && cells <= kSmallCells) {
         small_bins_kernel<<<1, 1024, 0, st>>>(x, y, n, static_cast<int>(cells), per, gv, gp ? w.grid : nullptr,
-                                              w.head, w.start, w.rank, w.sidx, w.sxy);
+                                              w.head, w.start, w.sidx, w.sxy);
         *launches += 1;
         return cudaGetLastError();
     }
@@ -1044,7 +1049,8 @@ QueryArgs query_args(const Workspace& w, const Grid* gp, const Grid& gv, int k, 
     a.k = k;
     a.ja = ja;
     a.status = &w.head->status;
-    a.undone = w.rank;  // ranks, none negative, no longer needed
+    a.list = w.rank;  // no longer needed
+    a.left = &w.head->left;
     // a block holds about 2 (k + 4 sqrt k) nodes; at 6.5 (k + 1) the dense-block
     // rule has taken the smaller block. Kept: k + 1 + 1.9 sqrt(k + 1) on average.
     a.cand_cap = (static_cast<int>(6.5 * (k + 1)) + 31) / 32 * 32;
@@ -1052,8 +1058,14 @@ QueryArgs query_args(const Workspace& w, const Grid* gp, const Grid& gv, int k, 
     return a;
 }
 
-// The nodes' own stencils over the binned nodes.
-cudaError_t enqueue_cells(const QueryArgs& a, size_t cells, bool periodic, int sms, cudaStream_t st) {
+// The nodes' own stencils over the binned nodes. A small set's cells are shared by
+// several warps, so that all the warps of the chip take part: 3,000 nodes of
+// fourfold varying density, us, one warp a cell and up to eight: k = 21 45 -> 35, k =
+// 35 70 -> 43, k = 61 125 -> 57; of a disk k = 61 70 -> 31. Up to 8,192 nodes about one
+// part a resident warp (two: 3,000 nodes of a square, k = 12, 30 us instead of 26),
+// above them two (25,000 nodes of varying density, k = 61: 110 us, one 163).
+constexpr int kMaxSplit = 8;
+cudaError_t enqueue_cells(QueryArgs a, size_t cells, bool periodic, int sms, cudaStream_t st) {
     const size_t smem = kWarps * cell_smem(a.cand_cap, a.keep_cap);
     void (*kern)(QueryArgs) = nullptr;
     if (a.keep_cap <= 96)
@@ -1067,9 +1079,13 @@ cudaError_t enqueue_cells(const QueryArgs& a, size_t cells, bool periodic, int s
                                                    static_cast<int>(smem));
         if (e != cudaSuccess) return e;
     }
-    const size_t want = (cells + kWarps - 1) / kWarps;
+    const size_t items = static_cast<size_t>(sms) * (a.nq <= kSmallNodes ? 24 : 48);
+    a.split = static_cast<int>(std::min<size_t>(kMaxSplit, std::max<size_t>(1, items / cells)));
+    const size_t want = (cells * a.split + kWarps - 1) / kWarps;
     const int blocks = static_cast<int>(std::max<size_t>(1, std::min<size_t>(want, sms * 64)));
     kern<<<blocks, kWarps * 32, smem, st>>>(a);
+    const int rest = static_cast<int>(std::min<size_t>((a.nq + kWarps - 1) / kWarps, sms * 8));
+    leftover_kernel<<<rest, kWarps * 32, 0, st>>>(a);
     return cudaGetLastError();
 }
 
@@ -1092,7 +1108,9 @@ int search(rbfb_ctx* ctx, int n, const double* x, const double* y, int nq, const
     ctx->launches += launches;
     QueryArgs a = query_args(w, gp, gv, k, ja);
     if (!xq) {
+        a.nq = n;
         RBFB_CUDA(ctx, enqueue_cells(a, cells, periodic, ctx->sms, st));
+        ctx->launches += 1;
     } else {
         if (nq == 0) return RBFB_OK;
         a.nq = nq;
@@ -1258,8 +1276,10 @@ extern "C" int rbfb_knn_stencils_static(int n, const double* x, const double* y,
     cudaStream_t st = static_cast<cudaStream_t>(stream);
     const Grid* gp = periodic ? nullptr : w.grid;
     int launches = 0;
+    QueryArgs a = query_args(w, gp, gv, k, ja);
+    a.nq = n;
     if (enqueue_bins(w, n, x, y, cells, per, gp, gv, sms, st, &launches) != cudaSuccess ||
-        enqueue_cells(query_args(w, gp, gv, k, ja), cells, periodic, sms, st) != cudaSuccess)
+        enqueue_cells(a, cells, periodic, sms, st) != cudaSuccess)
         return RBFB_ECUDA;
     return RBFB_OK;
 }

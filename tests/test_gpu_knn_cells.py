@@ -110,3 +110,13 @@ def test_either_side_of_the_one_block_binning(ctx, torch_cuda, make, n):
     x, y = make(np.random.default_rng(n), n)
     for k, period in ((21, None), (35, (2.0, 3.0))):
         _check(ctx, torch_cuda, x, y, k, period)
+
+
+# cells shared by up to eight warps, and by none; many nodes left over (a density
+# that varies a hundredfold)
+@pytest.mark.parametrize("n,k", [(70, 9), (400, 61), (3000, 35), (9000, 61), (20000, 21)])
+def test_shared_cells_and_leftovers(ctx, torch_cuda, n, k):
+    rng = np.random.default_rng(n + k)
+    r, t = rng.uniform(0, 1, n) ** 2, rng.uniform(0, 2 * np.pi, n)
+    for period in (None, (2.0, 2.0)):
+        _check(ctx, torch_cuda, r * np.cos(t), r * np.sin(t), k, period)
