@@ -24,7 +24,7 @@ Workloads:
             departure points x - c_a h/2, assembled once, then --reps fused
             stream + collide steps (populations in --populations precision)
 The single-kernel shapes are also what the profiles are captured on (e.g.
-under ncu with ``-k regex:asm_kernel`` on ``--grid 512``).
+under ncu with ``-k regex:dm_kernel`` on ``--grid 512``).
 
 --solve N (disk only) then runs N BiCGSTAB iterations (tolerance 0, so
 exactly N) on the assembled FP64 Laplacian with identity rows at the

@@ -133,7 +133,7 @@ int rbfb_knn_query(rbfb_ctx* ctx, int n, const double* x, const double* y, int n
  * host whose device memory belongs to another framework's allocator. No
  * counterpart in the reference (its searches run on the host).
  *
- * Needs no context: the scratch is a fixed array of about 3 MB in device
+ * Needs no context: the scratch is a fixed array of about 2.2 MB in device
  * memory, held by every GPU that loads this library until the process exits.
  * Limit: n <= 65,536 nodes (and a cell grid of at most n/2 cells); larger
  * problems are rejected with RBFB_ETOOBIG. The first call on a device looks
@@ -383,7 +383,7 @@ int rbfb_autotune(rbfb_ctx* ctx, const rbfb_desc* desc, int nstencils, const dou
                   const double* y, int k, const int* ja, double* const* values_h);
 
 /* Name of compiled kernel shape `index` (as returned by rbfb_autotune), e.g.
- * "mix_p3q5_n48_g16x2", or NULL past the last one. */
+ * "bmx_p3q5_n48_w1x9", or NULL past the last one. */
 const char* rbfb_variant_name(int index);
 
 /* Pins compiled shape `index` (and CTAs per SM, 0 = the occupancy maximum)
