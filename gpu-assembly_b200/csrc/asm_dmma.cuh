@@ -179,7 +179,7 @@ __device__ __forceinline__ double mul_pow2(double x, int e) {
 // power-of-two radius scale (src/rbf_operators.h:354-358), by one warp. With
 // PF xy holds the raw prefetched coordinates on entry. Returns the exponent.
 template <int KMAX, bool PF, bool CAREFUL>
-__device__ __forceinline__ int gather_scale(const AsmParams& p, int off, int ks, double x0,
+__device__ __forceinline__ int gather_scale(const AsmParams& p, long long off, int ks, double x0,
                                             double y0, double2* xy, int lane) {
     constexpr int KPL = (KMAX + 31) / 32;
     double gx[KPL], gy[KPL];
@@ -757,7 +757,7 @@ __device__ __forceinline__ int eliminate(double* S, uint8_t* lists, uint8_t* piv
 // the steps of the last block below cstop are taken but not written.
 template <int LDS, int NRHS, bool CAREFUL>
 __device__ __forceinline__ void back_substitute(const AsmParams& p, double* S, const uint8_t* piv,
-                                                int n, int cstop, int off, int e, int info,
+                                                int n, int cstop, long long off, int e, int info,
                                                 int lane) {
     constexpr unsigned ALL = 0xffffffffu;
     constexpr int SL = (NRHS + 3) / 4;  // right-hand sides a lane
@@ -878,7 +878,7 @@ __device__ __forceinline__ bool fill_shape(const AsmParams& p, Sh sh, double* S,
 // The careful path of one stencil, from its global data: everything the fast
 // path leaves out (coincident nodes, zero pivots, extreme magnitudes). Cold.
 template <class L, int NRHS, int NW, class Sh>
-__device__ __noinline__ void assemble_careful(const AsmParams& p, Sh sh, int s, int off, int ks,
+__device__ __noinline__ void assemble_careful(const AsmParams& p, Sh sh, int s, long long off, int ks,
                                               char* base, int warp, int lane) {
     constexpr int LDS = L::LDS;
     double2* xy = reinterpret_cast<double2*>(base + L::off_xy);
@@ -907,16 +907,19 @@ __device__ __noinline__ void assemble_careful(const AsmParams& p, Sh sh, int s, 
     stencil_sync<NW>();
 }
 
-// Stencil s: its offset in ja and the value arrays, its size, its centre.
+// Stencil s: its size, its offset in ja and the value arrays (in 64 bits: a
+// fixed-width batch may hold more than 2^31 entries), its centre.
 struct Item {
-    int s, off, ks;
+    int s, ks;
+    long long off;
     double x0, y0;
 };
 __device__ __forceinline__ Item item_of(const AsmParams& p, int s) {
-    Item it{s, (s - p.row_base) * p.k, p.k, __ldg(p.x + s), __ldg(p.y + s)};
+    Item it{s, p.k, static_cast<long long>(s - p.row_base) * p.k, __ldg(p.x + s), __ldg(p.y + s)};
     if (p.ia) {
-        it.off = __ldg(p.ia + s);
-        it.ks = __ldg(p.ia + s + 1) - it.off;
+        const int first = __ldg(p.ia + s);
+        it.off = first;
+        it.ks = __ldg(p.ia + s + 1) - first;
     }
     return it;
 }
