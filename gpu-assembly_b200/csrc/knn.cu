@@ -45,7 +45,11 @@ constexpr int kPerCell = 2;   // target nodes per cell for arbitrary query point
 constexpr int kCap = 256;     // candidate buffer per warp (entries)
 constexpr int kWarps = 4;     // warps per CTA in the query kernel
 constexpr int kMaxK = 128;
-constexpr int kMaxKeep = 320;  // largest list of kept candidates (keep_cap(kMaxK))
+// Capacities of a warp's lists for k neighbours: a block's candidates, and the
+// kept ones (k + 1 + 1.9 sqrt(k + 1) on average).
+__host__ __device__ constexpr int cand_cap_of(int k) { return (static_cast<int>(6.5 * (k + 1)) + 31) / 32 * 32; }
+__host__ __device__ constexpr int keep_cap_of(int k) { return (static_cast<int>(2.2 * (k + 1)) + 31) / 32 * 32; }
+constexpr int kMaxCand = cand_cap_of(kMaxK), kMaxKeep = keep_cap_of(kMaxK);
 
 struct Grid {
     double x0, y0;     // origin of the cell grid
@@ -1051,10 +1055,8 @@ QueryArgs query_args(const Workspace& w, const Grid* gp, const Grid& gv, int k, 
     a.status = &w.head->status;
     a.list = w.rank;  // no longer needed
     a.left = &w.head->left;
-    // a block holds about 2 (k + 4 sqrt k) nodes; at 6.5 (k + 1) the dense-block
-    // rule has taken the smaller block. Kept: k + 1 + 1.9 sqrt(k + 1) on average.
-    a.cand_cap = (static_cast<int>(6.5 * (k + 1)) + 31) / 32 * 32;
-    a.keep_cap = std::min(kMaxKeep, (static_cast<int>(2.2 * (k + 1)) + 31) / 32 * 32);
+    a.cand_cap = cand_cap_of(k);
+    a.keep_cap = keep_cap_of(k);
     return a;
 }
 
@@ -1075,8 +1077,10 @@ cudaError_t enqueue_cells(QueryArgs a, size_t cells, bool periodic, int sms, cud
     else
         kern = periodic ? &cell_query_kernel<true, kMaxKeep / 32> : &cell_query_kernel<false, kMaxKeep / 32>;
     if (smem > 48 * 1024) {
-        const cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                                   static_cast<int>(smem));
+        // the limit is the process's, not this call's: always the largest that a call
+        // can ask for, or another thread's launch would be refused
+        constexpr int most = static_cast<int>(kWarps * cell_smem(kMaxCand, kMaxKeep));
+        const cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, most);
         if (e != cudaSuccess) return e;
     }
     const size_t items = static_cast<size_t>(sms) * (a.nq <= kSmallNodes ? 24 : 48);

@@ -189,6 +189,7 @@ __global__ void bgk_kernel(int n, T omega, T* __restrict__ pdf, T* __restrict__ 
     }
 }
 
+constexpr int kMaxStencil = 64;  // largest stencil of a streaming step
 constexpr int kTileWarps = 4;  // warps a CTA; each warp owns a 32-node tile at a time
 
 // How a tile's rows are copied into its slabs: in 16-byte pieces of one run, in
@@ -343,11 +344,16 @@ template <typename T, int COPY, int KT>
 int launch_stream_collide(int n, int k, const int* ja, const double* W, T omega, const T* pin,
                           T* pout, T* rho, T* ux, T* uy, cudaStream_t st) {
     auto kern = stream_collide_kernel<T, COPY, KT>;
-    const size_t smem = static_cast<size_t>(kTileWarps) * 32 *
-                        (2 * weight_stride<COPY>(k) * sizeof(double) +
-                         (KT ? 0 : index_stride<COPY>(k) * sizeof(int)));
+    auto bytes = [](int rows_of) {
+        return static_cast<size_t>(kTileWarps) * 32 *
+               (2 * weight_stride<COPY>(rows_of) * sizeof(double) +
+                (KT ? 0 : index_stride<COPY>(rows_of) * sizeof(int)));
+    };
+    const size_t smem = bytes(k);
+    // the limit is the process's, not this call's: always the largest that a call can
+    // ask for, or another thread's launch would be refused
     if (cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                             static_cast<int>(smem)) != cudaSuccess)
+                             static_cast<int>(bytes(KT ? k : kMaxStencil))) != cudaSuccess)
         return RBFB_ECUDA;
     int dev = 0, sms = 0, per_sm = 0;
     cudaGetDevice(&dev);
@@ -463,7 +469,7 @@ int rbfb_lbm_bgk(int n, int precision, double omega, void* pdf, void* rho, void*
 int rbfb_lbm_stream_collide(int n, int precision, int k, const int* ja, const double* W,
                             double omega, const void* pdf_in, void* pdf_out, void* rho, void* ux,
                             void* uy, void* stream) {
-    if (n < 0 || k < 1 || k > 64 || !ja || !W || !pdf_in || !pdf_out || pdf_in == pdf_out)
+    if (n < 0 || k < 1 || k > kMaxStencil || !ja || !W || !pdf_in || !pdf_out || pdf_in == pdf_out)
         return RBFB_EINVAL;
     if (n == 0) return RBFB_OK;
     cudaStream_t st = static_cast<cudaStream_t>(stream);

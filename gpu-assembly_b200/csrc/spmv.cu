@@ -119,8 +119,11 @@ int launch_spmv(int n, int k, const int* ja, const double* values, const double*
     const int warps = k < 60 && static_cast<long long>(n) * k * 12 <= kL2Bytes ? 1 : kSpmvWarps;
     const size_t smem = warps * t.warp_bytes();
     auto* kern = k % 4 == 0 ? &spmv_tiled_kernel<true> : &spmv_tiled_kernel<false>;
+    // the limit is the process's, not this call's: always the largest that a call can
+    // ask for, or another thread's launch would be refused
+    const size_t most = kSpmvWarps * tile_shape(kTiledMaxK).warp_bytes();
     if (smem > 48 * 1024 && cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                                 static_cast<int>(smem)) != cudaSuccess)
+                                                 static_cast<int>(most)) != cudaSuccess)
         return RBFB_ECUDA;
     const int per_block = warps * t.rows;
     const int blocks = std::min((n + per_block - 1) / per_block, 148 * 256 / warps);
