@@ -457,8 +457,9 @@ __device__ __forceinline__ void block8(const float* s, float* u) {
 }
 
 // y = L^-1 y in place (unit lower factors), blocks of 8 steps in order. The
-// blocks from nt on take part (in values that nothing reads) rather than a
-// branch each, which would keep the chains of one block from overlapping.
+// blocks from nt on take part rather than a branch each, which would keep the
+// chains of one block from overlapping: their entries of y hold no unknown
+// afterwards, nor do those past n in the last block.
 template <int NT>
 __device__ __forceinline__ void forward(const float* S, const int (&prow)[NT], float (&y)[NT], int nt,
                                         int lane) {
@@ -613,8 +614,9 @@ __device__ __forceinline__ void assemble(const AsmParams& p, const Item& it, con
         uint32_t dmax = 0, xmax = 0;
 #pragma unroll
         for (int t = 0; t < NT; ++t) {
-            x[t] = x[t] + (double)y[t];
-            dmax = max(dmax, __float_as_uint(fabsf(y[t])));
+            const float d = 8 * t + g < n ? y[t] : 0.f;  // only unknowns count
+            x[t] = x[t] + (double)d;
+            dmax = max(dmax, __float_as_uint(fabsf(d)));
             xmax = max(xmax, __float_as_uint(fabsf((float)x[t])));
         }
 #pragma unroll
