@@ -68,6 +68,14 @@ constexpr int kVectorBlocksPerSm = 4, kUpdateBlocksPerSm = 3;
 // iterations: 11.9 ms; three blocks of 768 entries 13.8, four of 576 15.2).
 constexpr int kStageEntries = 1024;
 constexpr int kStagedBlocksPerSm = 2;
+// Rows whose first entries lie a multiple of 16 apart start in the same bank, and
+// the lanes, in step through their rows, meet there for every entry. When more
+// than kMostClashing of a warp's rows share the first one's bank (rows of 8, 16, 24, ...
+// entries), the rows are walked from global memory instead. us an iteration,
+// 32,000 / 600,000 rows, staged and walked: k = 16 29 / 154 and 23 / 112, k = 32 51 /
+// 330 and 32 / 172, k = 48 57 / 377 and 38 / 246, k = 64 87 / 610 and 46 / 300; k = 12, 20
+// (a quarter of the lanes) 20 / 82 and 21 / 89, 22 / 105 and 24 / 130.
+constexpr int kMostClashing = 8;
 constexpr size_t kStageBytes = static_cast<size_t>(kWarps) * kStageEntries * (sizeof(double) + sizeof(int));
 
 enum : int { RUNNING = 0, CONVERGED = 1, MAXIT = 2, BREAKDOWN = 3, ZERO_RHS = 4, BAD_INPUT = 5 };
@@ -130,8 +138,9 @@ __device__ __forceinline__ double apply_row(const Args& a, long long s, W w) {
 // boundary) are copied into the warp's shared-memory slab with 16-byte
 // copies under an L2 evict-first policy, and each lane sums its own row from
 // there (eight gathers of w in flight; sixteen measured
-// slower). A piece above kStageEntries (or unaligned arrays) is walked from
-// global memory by row_sum. Same rows, same order, same sums as apply_row.
+// slower). A piece above kStageEntries, unaligned arrays and rows that meet in a
+// bank (kMostClashing) are walked from global memory by row_sum. Same rows, same
+// order, same sums as apply_row.
 //
 // The first rows' entries are requested before ready() is called: it waits for
 // the kernel's predecessor, and returns false when there is nothing to do.
@@ -158,14 +167,19 @@ __device__ __forceinline__ bool walk_rows(const Args& a, unsigned char* smem, R 
             e = q + a.k;
         }
         const bool bnd = a.bflag[sc];
-        for (int r0 = 0, rows = 32; r0 < 32 && t0 + r0 < a.n; r0 += rows) {
+        const long long w0 = __shfl_sync(0xffffffffu, q, 0), w1 = __shfl_sync(0xffffffffu, e, 31);
+        const bool clash = s < a.n && ((q - w0) & 15) == 0;
+        bool staged = a.vec && __popc(__ballot_sync(0xffffffffu, clash)) <= kMostClashing;
+        // all 32 rows at once, or 16 at a time where that lets both pieces fit
+        int rows = 32;
+        if (staged && w1 - (w0 & ~3LL) > kStageEntries) {
+            const long long h0 = __shfl_sync(0xffffffffu, q, 16), h1 = __shfl_sync(0xffffffffu, e, 15);
+            staged = h1 - (w0 & ~3LL) <= kStageEntries && w1 - (h0 & ~3LL) <= kStageEntries;
+            rows = staged ? 16 : 32;
+        }
+        for (int r0 = 0; r0 < 32 && t0 + r0 < a.n; r0 += rows) {
             const long long qa = __shfl_sync(0xffffffffu, q, r0) & ~3LL;
-            long long q1 = __shfl_sync(0xffffffffu, e, r0 + rows - 1);
-            if (rows == 32 && q1 - qa > kStageEntries) {
-                rows = 16;
-                q1 = __shfl_sync(0xffffffffu, e, 15);
-            }
-            const bool staged = a.vec && q1 - qa <= kStageEntries;
+            const long long q1 = __shfl_sync(0xffffffffu, e, r0 + rows - 1);
             if (staged) {
                 const int m = static_cast<int>(q1 - qa);
                 const double* gv = a.values + qa;
