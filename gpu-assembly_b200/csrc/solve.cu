@@ -77,6 +77,12 @@ constexpr int kStagedBlocksPerSm = 2;
 // (a quarter of the lanes) 20 / 82 and 21 / 89, 22 / 105 and 24 / 130.
 constexpr int kMostClashing = 8;
 constexpr size_t kStageBytes = static_cast<size_t>(kWarps) * kStageEntries * (sizeof(double) + sizeof(int));
+// What a block asks for instead when the grid has no more blocks than the chip has
+// SMs: more than half of an SM. The blocks start while those of the pass before
+// still hold most SMs, and two at a time would fill the free ones: half the chip
+// idle, up to twice the time of a pass. us an iteration, 32,000 rows (125 blocks)
+// of 80, 64, 48 and 21 entries: 51, 46, 38 and 20 two to an SM, 34, 32, 28 and 20 alone.
+constexpr size_t kAloneBytes = 116 * 1024;
 
 enum : int { RUNNING = 0, CONVERGED = 1, MAXIT = 2, BREAKDOWN = 3, ZERO_RHS = 4, BAD_INPUT = 5 };
 
@@ -583,9 +589,9 @@ int ensure(rbfb_ctx* ctx, int n, int grid) {
         RBFB_CUDA(ctx, cudaMallocHost(&w->st_h, sizeof(State)));
         // the operator passes' staging slabs (above the 48 KB default)
         RBFB_CUDA(ctx, cudaFuncSetAttribute(spmv_v_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                            static_cast<int>(kStageBytes)));
+                                            static_cast<int>(kAloneBytes)));
         RBFB_CUDA(ctx, cudaFuncSetAttribute(spmv_t_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                            static_cast<int>(kStageBytes)));
+                                            static_cast<int>(kAloneBytes)));
     }
     if (static_cast<size_t>(n) > w->cap) {
         if (w->graph) cudaGraphExecDestroy(w->graph);
@@ -634,11 +640,12 @@ cudaError_t launch(void (*kern)(Args), int grid, size_t smem, cudaStream_t st, c
 
 // Enqueues kChunk iterations (5 launches each).
 int enqueue_chunk(rbfb_ctx* ctx, const Args& a, int grid, cudaStream_t st) {
+    const size_t smem = grid <= ctx->sms ? kAloneBytes : kStageBytes;
     for (int it = 0; it < kChunk; ++it) {
         RBFB_CUDA(ctx, launch(p_kernel, grid, 0, st, a));
-        RBFB_CUDA(ctx, launch(spmv_v_kernel, grid, kStageBytes, st, a));
+        RBFB_CUDA(ctx, launch(spmv_v_kernel, grid, smem, st, a));
         RBFB_CUDA(ctx, launch(s_kernel, grid, 0, st, a));
-        RBFB_CUDA(ctx, launch(spmv_t_kernel, grid, kStageBytes, st, a));
+        RBFB_CUDA(ctx, launch(spmv_t_kernel, grid, smem, st, a));
         RBFB_CUDA(ctx, launch(update_kernel, grid, 0, st, a));
         ctx->launches += 5;
     }

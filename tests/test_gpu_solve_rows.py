@@ -83,3 +83,11 @@ def test_rows_that_meet_in_a_bank_are_not_slower(ctx, torch_cuda, n, k):
     """A 16-fold conflict would cost 2.5 times the next shorter row."""
     times = sorted(_iteration_s(ctx, torch_cuda, n, k) / _iteration_s(ctx, torch_cuda, n, k - 1) for _ in range(3))
     assert times[1] < 1.6
+
+
+def test_few_blocks_spread_over_the_chip(ctx, torch_cuda):
+    """32,000 rows are one block for most SMs. Two blocks on an SM and none on
+    another would take 0.45 of the time of 150,000 rows, one on each takes 0.3."""
+    T = torch_cuda
+    times = sorted(_iteration_s(ctx, T, 32000, 95) / _iteration_s(ctx, T, 150000, 95) for _ in range(3))
+    assert times[1] < 0.38
