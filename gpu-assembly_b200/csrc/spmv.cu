@@ -90,7 +90,7 @@ __global__ void __launch_bounds__(kSpmvWarps * 32, 8)
     }
 }
 
-// Unaligned arrays and very long rows: one thread per row (row_sum).
+// Unaligned arrays, short and very long rows: one thread per row (row_sum).
 __global__ void spmv_fixed_kernel(int n, int k, const int* __restrict__ ja,
                                   const double* __restrict__ values, const double* __restrict__ u,
                                   double* __restrict__ out, bool vec) {
@@ -100,31 +100,35 @@ __global__ void spmv_fixed_kernel(int n, int k, const int* __restrict__ ja,
     }
 }
 
-constexpr int kTiledMaxK = 128;  // above: the slabs leave too few warps
+// Rows that go by tiles. Shorter ones: a tile is a few hundred bytes, and its fixed cost
+// stays (k = 4, 1M rows: 22 us a tile of 32 rows at a time, 11.2 us a thread a row; k =
+// 8 24 and 22; k = 9 25 and 36); the padded rows of 12 entries only beyond L2 (400,000 rows
+// 15.4 and 13.1, 800,000 26 and 31). Longer ones: the slabs leave too few warps.
+constexpr int kTiledMinK = 9, kTiledMaxK = 128;
 constexpr long long kL2Bytes = 126ll * 1000 * 1000;
+
+bool by_tiles(int n, int k) {
+    if (k == 12) return static_cast<long long>(n) * k * 12 > kL2Bytes / 4 * 3;
+    return k >= kTiledMinK && k <= kTiledMaxK;
+}
 
 int launch_spmv(int n, int k, const int* ja, const double* values, const double* u, double* out,
                 cudaStream_t st) {
     const bool vec = rows_vectorizable(ja, values);
-    if (!vec || k > kTiledMaxK) {
+    if (!vec || !by_tiles(n, k)) {
         const int blocks = std::min((n + 255) / 256, 148 * 16);
         spmv_fixed_kernel<<<blocks, 256, 0, st>>>(n, k, ja, values, u, out, vec);
         return RBFB_OK;
     }
     const TileShape t = tile_shape(k);
     // Blocks of one warp even out the last wave, which counts while the operator
-    // comes from L2 (k = 35, 150,000 rows: 15.2 us, four warps 17.9); beyond it, and
-    // for the few warps that long rows leave, four are as good or better (k = 44,
-    // 700,000 rows: 80 against 84; k = 60, 60,000 rows: 14.5 against 15.9).
-    const int warps = k < 60 && static_cast<long long>(n) * k * 12 <= kL2Bytes ? 1 : kSpmvWarps;
-    const size_t smem = warps * t.warp_bytes();
+    // comes from L2 (k = 35, 150,000 rows: 15.2 us, four warps 17.9), and for long rows, of
+    // which an SM holds few blocks of four (k = 100, 60,000 rows: 22.0 us against 26.4; 600,000:
+    // 176 against 210; k = 60, 60,000 rows: 14.1 and 14.2). Beyond L2 four are as good or better
+    // for the others (k = 44, 700,000 rows: 80 us against 84).
+    const int warps = k >= 60 || static_cast<long long>(n) * k * 12 <= kL2Bytes ? 1 : kSpmvWarps;
+    const size_t smem = warps * t.warp_bytes();  // at most 45.5 KB
     auto* kern = k % 4 == 0 ? &spmv_tiled_kernel<true> : &spmv_tiled_kernel<false>;
-    // the limit is the process's, not this call's: always the largest that a call can
-    // ask for, or another thread's launch would be refused
-    const size_t most = kSpmvWarps * tile_shape(kTiledMaxK).warp_bytes();
-    if (smem > 48 * 1024 && cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                                 static_cast<int>(most)) != cudaSuccess)
-        return RBFB_ECUDA;
     const int per_block = warps * t.rows;
     const int blocks = std::min((n + per_block - 1) / per_block, 148 * 256 / warps);
     kern<<<blocks, warps * 32, smem, st>>>(n, k, t, ja, values, u, out);
