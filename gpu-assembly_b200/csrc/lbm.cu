@@ -208,9 +208,22 @@ __host__ __device__ inline int index_stride(int k) {
     return COPY == kRows16 ? (k / 4 % 2 ? k : k + 4) : COPY == kPad8 ? k + 1 : k;
 }
 
-// Copies the tile's m entries of rows of k into a slab of stride ks.
+// A lane's walk over the pieces of rows that are copied row by row: its first
+// piece's row and place in the row, and the step of 32 pieces (formed once a warp: the
+// divisions cost more than a short row's copy).
+struct Pieces {
+    int row, r, c, dr, dc;
+};
 template <int COPY, typename V>
-__device__ __forceinline__ void copy_slab(V* dst, const V* src, int m, int k, int ks, int lane,
+__device__ __forceinline__ Pieces pieces(int k, int lane) {
+    const int row = COPY == kRows16 ? k / (16 / static_cast<int>(sizeof(V))) : k;
+    const int r = lane / row, dr = 32 / row;
+    return {row, r, lane - r * row, dr, 32 - dr * row};
+}
+
+// Copies the tile's m entries into a slab, rows ks entries apart.
+template <int COPY, typename V>
+__device__ __forceinline__ void copy_slab(V* dst, const V* src, int m, const Pieces& p, int ks, int lane,
                                           unsigned long long pol) {
     constexpr int per = 16 / sizeof(V);
     if constexpr (COPY == kRun16) {
@@ -219,16 +232,17 @@ __device__ __forceinline__ void copy_slab(V* dst, const V* src, int m, int k, in
             cp_async_stream<16>(dst + q * per, src + q * per, pol);
         for (int e = chunks * per + lane; e < m; e += 32)
             cp_async_stream<sizeof(V)>(dst + e, src + e, pol);
+    } else if constexpr (COPY == kRun8) {
+        for (int q = lane; q < m; q += 32) cp_async_stream<sizeof(V)>(dst + q, src + q, pol);
     } else {
         constexpr int step = COPY == kRows16 ? per : 1;
-        const int row = k / step, q32 = 32 / row, r32 = 32 - q32 * row;
-        int r = lane / row, c = lane - r * row;  // of this lane's piece
+        int r = p.r, c = p.c;
         for (int q = lane; q < m / step; q += 32) {
             cp_async_stream<step * sizeof(V)>(dst + r * ks + c * step, src + q * step, pol);
-            r += q32;
-            c += r32;
-            if (c >= row) {
-                c -= row;
+            r += p.dr;
+            c += p.dc;
+            if (c >= p.row) {
+                c -= p.row;
                 ++r;
             }
         }
@@ -259,13 +273,18 @@ __device__ __forceinline__ void copy_slab(V* dst, const V* src, int m, int k, in
 // gathers in flight are worth more than more warps. 1M nodes, k = 15 187 (6) and
 // 195 us (4), k = 16 223 and 209, k = 21 254 and 248; left to itself the compiler
 // takes 56 registers for k = 21 in FP32, 330 us against 229.
-constexpr int resident(int kt, int stride) {
+// KT = kShort: any k of a few entries. The batch of eight gathers, most of it
+// predicated off, and its 100 registers cost such rows up to 1.75 times the time of a plain
+// loop: FP64, 600,000 nodes, k = 1 33 against 57 us, k = 9 (odd n) 86 and 109. As many CTAs
+// as 64 registers (FP32: 40) allow.
+constexpr int kShort = -1;
+constexpr int resident(int kt, int stride, bool fp32) {
     const int fit = 227 * 1024 / (kTileWarps * 32 * 2 * stride * 8 + 1024);
     const int most = kt > 0 && kt < 16 ? 6 : 4;
-    return kt == 0 ? most : fit < most ? fit : most;
+    return kt == kShort ? (fp32 ? 12 : 8) : kt == 0 ? most : fit < most ? fit : most;
 }
 template <typename T, int COPY, int KT>
-__global__ void __launch_bounds__(kTileWarps * 32, resident(KT, weight_stride<COPY>(KT)))
+__global__ void __launch_bounds__(kTileWarps * 32, resident(KT, weight_stride<COPY>(KT), sizeof(T) == 4))
     stream_collide_kernel(
     int n, int k, const int* __restrict__ ja, const double* __restrict__ W, T omega,
     const T* __restrict__ pdf_in, T* __restrict__ pdf_out, T* __restrict__ rho,
@@ -276,23 +295,24 @@ __global__ void __launch_bounds__(kTileWarps * 32, resident(KT, weight_stride<CO
     const int kv = weight_stride<COPY>(k), kj = index_stride<COPY>(k);
     const int slab = 32 * kv;
     double* wbuf = reinterpret_cast<double*>(tile_smem) + static_cast<size_t>(wid) * 2 * slab;
-    int* jbuf = KT ? reinterpret_cast<int*>(wbuf + slab)
-                   : reinterpret_cast<int*>(reinterpret_cast<double*>(tile_smem) +
-                                            static_cast<size_t>(kTileWarps) * 2 * slab) +
-                         static_cast<size_t>(wid) * 32 * kj;
+    int* jbuf = KT > 0 ? reinterpret_cast<int*>(wbuf + slab)
+                       : reinterpret_cast<int*>(reinterpret_cast<double*>(tile_smem) +
+                                                static_cast<size_t>(kTileWarps) * 2 * slab) +
+                             static_cast<size_t>(wid) * 32 * kj;
     const size_t N = static_cast<size_t>(n);
     const size_t nnz = N * static_cast<size_t>(k);
     const unsigned long long pol = evict_first_policy();
+    const Pieces pw = pieces<COPY, double>(k, lane), pj = pieces<COPY, int>(k, lane);
     const int tiles = (n + 31) >> 5;
     for (int tile = blockIdx.x * kTileWarps + wid; tile < tiles; tile += gridDim.x * kTileWarps) {
         const int s0 = tile << 5;
         const int cnt = min(32, n - s0);
         const int m = cnt * k;
         const size_t base = static_cast<size_t>(s0) * k;
-        copy_slab<COPY>(jbuf, ja + base, m, k, kj, lane, pol);
-        copy_slab<COPY>(wbuf, W + base, m, k, kv, lane, pol);
+        copy_slab<COPY>(jbuf, ja + base, m, pj, kj, lane, pol);
+        copy_slab<COPY>(wbuf, W + base, m, pw, kv, lane, pol);
         cp_async_commit();
-        int jrow[KT ? KT : 1];
+        int jrow[KT > 0 ? KT : 1];
         if constexpr (KT > 0) {  // the lane's index row, then the slab is free
             cp_async_wait<0>();
             __syncwarp();
@@ -305,7 +325,7 @@ __global__ void __launch_bounds__(kTileWarps * 32, resident(KT, weight_stride<CO
 #pragma unroll
         for (int a = 1; a < 9; ++a) {
             if (a < 8) {
-                copy_slab<COPY>(wbuf + (a & 1) * slab, W + static_cast<size_t>(a) * nnz + base, m, k, kv,
+                copy_slab<COPY>(wbuf + (a & 1) * slab, W + static_cast<size_t>(a) * nnz + base, m, pw, kv,
                                 lane, pol);
                 cp_async_commit();
             }
@@ -318,6 +338,12 @@ __global__ void __launch_bounds__(kTileWarps * 32, resident(KT, weight_stride<CO
                     T v = mul(static_cast<T>(wr[0]), pa[jrow[0]]);
 #pragma unroll
                     for (int j = 1; j < KT; ++j) v = fmaT(static_cast<T>(wr[j]), pa[jrow[j]], v);
+                    f[a] = v;
+                } else if constexpr (KT == kShort) {
+                    const int* jr = jbuf + lane * kj;
+                    T v = mul(static_cast<T>(wr[0]), pa[jr[0]]);
+#pragma unroll 8
+                    for (int j = 1; j < k; ++j) v = fmaT(static_cast<T>(wr[j]), pa[jr[j]], v);
                     f[a] = v;
                 } else {
                     // a sum from -0 gives the first product itself
@@ -347,13 +373,13 @@ int launch_stream_collide(int n, int k, const int* ja, const double* W, T omega,
     auto bytes = [](int rows_of) {
         return static_cast<size_t>(kTileWarps) * 32 *
                (2 * weight_stride<COPY>(rows_of) * sizeof(double) +
-                (KT ? 0 : index_stride<COPY>(rows_of) * sizeof(int)));
+                (KT > 0 ? 0 : index_stride<COPY>(rows_of) * sizeof(int)));
     };
     const size_t smem = bytes(k);
     // the limit is the process's, not this call's: always the largest that a call can
     // ask for, or another thread's launch would be refused
     if (cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                             static_cast<int>(bytes(KT ? k : kMaxStencil))) != cudaSuccess)
+                             static_cast<int>(bytes(KT > 0 ? k : kMaxStencil))) != cudaSuccess)
         return RBFB_ECUDA;
     int dev = 0, sms = 0, per_sm = 0;
     cudaGetDevice(&dev);
@@ -390,6 +416,15 @@ int stream_collide(int n, int k, const int* ja, const double* W, T omega, const 
                      ((static_cast<long long>(n) * k) & 1) == 0;
     if (vec && k >= kMinFixed && k <= kMaxFixed)
         return launch_fixed<T, kMinFixed>(n, k, ja, W, omega, pin, pout, rho, ux, uy, st);
+    // rows that are short and have no kernel of their size (fewer than kMinFixed entries, or
+    // an odd n k): FP32 9 entries are better off with the batches (33 us against 36)
+    if (k <= (sizeof(T) == 4 ? 8 : 10)) {
+        if (k % 2 == 0 && (k > 2 || sizeof(T) == 8))
+            return launch_stream_collide<T, kPad8, kShort>(n, k, ja, W, omega, pin, pout, rho, ux, uy, st);
+        if (vec)
+            return launch_stream_collide<T, kRun16, kShort>(n, k, ja, W, omega, pin, pout, rho, ux, uy, st);
+        return launch_stream_collide<T, kRun8, kShort>(n, k, ja, W, omega, pin, pout, rho, ux, uy, st);
+    }
     if (vec && k % 4 == 0)
         return launch_stream_collide<T, kRows16, 0>(n, k, ja, W, omega, pin, pout, rho, ux, uy, st);
     if (vec) return launch_stream_collide<T, kRun16, 0>(n, k, ja, W, omega, pin, pout, rho, ux, uy, st);
