@@ -659,12 +659,46 @@ __global__ void __launch_bounds__(kWarps * 32, 8) leftover_kernel(QueryArgs a) {
 
 // ---- the nodes' own stencils, cell by cell ------------------------------------
 constexpr int kBuckets = 128;  // of the counting sort: four a lane
+// Entries of a bucket that a lane compares its own with one after another. Above,
+// the distances are far from uniform over the circle (a tight cluster in a wide
+// circle), and all entries are compared with all.
+constexpr int kCrowded = 16;
 
 // Shared memory of one warp: the block's candidates (coordinates, node
 // indices), the kept ones (distance, node index) and the buckets.
 __host__ __device__ constexpr size_t cell_smem(int cand_cap, int keep_cap) {
     return (static_cast<size_t>(cand_cap) * 20 + static_cast<size_t>(keep_cap) * 12 +
             (kBuckets + 4) * 4 + 15) & ~size_t(15);
+}
+
+// Writes the indices of the k first of the `have` entries (kd: bits of the squared distance,
+// ki: node index) in the order (distance, index) to row: every entry compared
+// with all, four entries a lane at a time.
+__device__ __forceinline__ void rank_pairs(const unsigned long long* kd, const int* ki, int have, int k,
+                                           int* row, int lane) {
+    __syncwarp();
+    for (int c0 = lane; c0 - lane < have; c0 += 128) {
+        unsigned long long d[4];
+        int id[4], rank[4];
+#pragma unroll
+        for (int s = 0; s < 4; ++s) {
+            const int c = min(c0 + 32 * s, have - 1);
+            d[s] = kd[c];
+            id[s] = ki[c];
+            rank[s] = 0;
+        }
+#pragma unroll 4
+        for (int i = 0; i < have; ++i) {
+            const unsigned long long o = kd[i];
+            const int io = ki[i];
+#pragma unroll
+            for (int s = 0; s < 4; ++s) rank[s] += key_less(o, io, d[s], id[s]);
+        }
+#pragma unroll
+        for (int s = 0; s < 4; ++s)
+            if (c0 + 32 * s < have && rank[s] < k) row[rank[s]] = id[s];
+    }
+    __syncwarp();
 }
 
 // Ranks the `have` kept entries (kd: bits of the squared distance, ki: node
@@ -695,6 +729,10 @@ __device__ __forceinline__ void rank_kept(unsigned long long* kd, int* ki, int* 
     __syncwarp();
     {
         const int4 h = reinterpret_cast<const int4*>(hist)[lane];
+        if (__any_sync(0xffffffffu, max(max(h.x, h.y), max(h.z, h.w)) > kCrowded)) {
+            rank_pairs(kd, ki, have, k, row, lane);
+            return;
+        }
         const int own = h.x + h.y + h.z + h.w;
         int incl = own;
 #pragma unroll
@@ -875,6 +913,10 @@ __global__ void __launch_bounds__(kWarps * 32, NSMAX > 5 ? 6 : 8) cell_query_ker
                     // (a block that covers the whole domain bounds nothing)
                     const double bound2 = bound >= 1e299 ? INFINITY : bound > 0.0 ? bound * bound : 0.0;
                     double keep2 = bound2 < est2 ? bound2 : est2;
+                    // a radius that keeps too few or too many entries changes by the
+                    // density found, between the last that kept too few and the last
+                    // that kept too many
+                    float few = 0.f, many = INFINITY;
                     int have = 0;
                     for (int attempt = 0;; ++attempt) {
                         have = 0;
@@ -897,13 +939,16 @@ __global__ void __launch_bounds__(kWarps * 32, NSMAX > 5 ? 6 : 8) cell_query_ker
                             have += __popc(bal);
                         }
                         __syncwarp();
-                        if (attempt >= 3) break;
-                        if (have > a.keep_cap)
-                            keep2 = fmin(keep2, est2) * (1.4 * (k + 1) / have);
-                        else if (have < k && keep2 < bound2)
-                            keep2 = attempt < 1 ? fmin(bound2, 2.0 * est2) : bound2;
+                        const bool over = have > a.keep_cap;
+                        if ((have >= k && !over) || attempt >= 5 || (!over && keep2 >= bound2)) break;
+                        const float grow = fminf(4.f, 1.4f * (k + 1) / fmaxf(have, 1.f));
+                        if (over)
+                            many = static_cast<float>(keep2);
                         else
-                            break;
+                            few = static_cast<float>(keep2);
+                        double next = keep2 * (over ? grow : fmaxf(1.5f, grow));
+                        if (!(next > few && next < many)) next = 0.5f * (few + many);
+                        keep2 = next < bound2 ? next : bound2;
                     }
                     if (have < k || have > a.keep_cap) {
                         failed |= 1u << i;
