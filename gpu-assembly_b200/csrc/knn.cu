@@ -379,26 +379,18 @@ __device__ __forceinline__ bool key_less(unsigned long long da, int ia, unsigned
 }
 
 // The general search: the k nearest nodes of (qx, qy), query number q, by one
-// warp with kCap entries of scratch (d, id).
+// warp with kCap entries of scratch (d, id). It starts with the block of R rings
+// of cells around the query's cell, and there with the radius (squared) est2, which
+// only has to be a good guess: when fewer than k nodes lie inside, a wider one
+// follows, up to the block's own bound, then a larger block.
 __device__ __forceinline__ void search_one(const QueryArgs& a, const Grid& g, double qx, double qy,
-                                           int q, unsigned long long* d, int* id, int lane) {
+                                           int q, int R, double est2, unsigned long long* d, int* id,
+                                           int lane) {
     const int k = a.k;
     const int ccx = cell_coord(qx, g.x0, g.hx, g.cx);
     const int ccy = cell_coord(qy, g.y0, g.hy, g.cy);
-    int R = 1;
-    // initial ring from the density
-    {
-        const double want = (k + 1.0) / g.per;
-        R = max(1, (int)ceil(0.5 * (sqrt(want * 1.27) - 1.0)) + 1);
-    }
     bool done = false;
-    // First try a tighter radius than the block bound: the distance at
-    // which k + 1 nodes are expected at the grid's mean density (g.per
-    // per cell), with a 30% margin. Exactness does not depend on it: if
-    // fewer than k nodes lie inside, the block is walked again with the
-    // full bound.
-    const double est2 = 1.69 * (k + 1) * g.hx * g.hy / (3.141592653589793 * g.per);
-    bool tight = true;
+    double reach = est2;
     for (int attempt = 0; attempt < 64 && !done; ++attempt) {
         // periodic axes: never more than one period (no cell twice); open
         // axes: up to the whole grid (the clamp below keeps it in range)
@@ -443,7 +435,7 @@ __device__ __forceinline__ void search_one(const QueryArgs& a, const Grid& g, do
         // widens to the bound, then the block grows. (A block that covers
         // the whole domain keeps everything.)
         const double bound2 = bound >= 1e299 ? INFINITY : (bound > 0.0 ? bound * bound : 0.0);
-        const double keep2 = tight ? fmin(bound2, est2) : bound2;
+        double keep2 = fmin(bound2, reach);
         // gather candidates chunk by chunk; the current best k stay at the front.
         // The block is a list of runs of consecutive cells (one per row, two
         // where a periodic row wraps). A batch of up to 32 runs is laid out
@@ -546,6 +538,8 @@ __device__ __forceinline__ void search_one(const QueryArgs& a, const Grid& g, do
                             id[keepd[u]] = ti[u];
                         }
                     __syncwarp();
+                    // nothing farther than the k-th found so far is needed
+                    if (have >= k) keep2 = __longlong_as_double((long long)(d[k - 1] + 1));
                     have = min(have, k);
                 }
                 const int pos = have + __popc(bal & ((1u << lane) - 1u));
@@ -559,8 +553,8 @@ __device__ __forceinline__ void search_one(const QueryArgs& a, const Grid& g, do
             }
         }
         if (total < k) {
-            if (tight && keep2 < bound2) {
-                tight = false;  // same block, full bound
+            if (reach < bound2) {  // same block, a wider radius, then the full bound
+                reach = reach > est2 ? INFINITY : 4.0 * est2;
                 continue;
             }
             R += max(1, R / 2);
@@ -626,6 +620,16 @@ __device__ __forceinline__ void search_one(const QueryArgs& a, const Grid& g, do
     if (!done && lane == 0) atomicExch(a.status, 1);
 }
 
+// Where the general search starts at a density of `per` nodes a cell: the rings of
+// cells around the query's, and the radius (squared) at which k + 1 nodes are
+// expected, with a 30 % margin.
+__device__ __forceinline__ int rings_at(int k, double per) {
+    return max(1, (int)ceil(0.5 * (sqrt((k + 1.0) / per * 1.27) - 1.0)) + 1);
+}
+__device__ __forceinline__ double radius2_at(int k, const Grid& g, double per) {
+    return 1.69 * (k + 1) * g.hx * g.hy / (3.141592653589793 * per);
+}
+
 // Arbitrary query points, one warp each. Bounded to 8 CTAs (32 warps) per SM:
 // 64 registers and a few spilled bytes instead of 96 registers and about 20
 // warps; the search is issue-bound, and the extra warps fill the issue slots
@@ -635,8 +639,10 @@ __global__ void __launch_bounds__(kWarps * 32, 8) query_kernel(QueryArgs a) {
     __shared__ int si[kWarps][kCap];
     const int w = threadIdx.x >> 5, lane = threadIdx.x & 31;
     const Grid g = a.g ? *a.g : a.gv;
+    const int R = rings_at(a.k, g.per);
+    const double est2 = radius2_at(a.k, g, g.per);
     for (int q = blockIdx.x * kWarps + w; q < a.nq; q += gridDim.x * kWarps)
-        search_one(a, g, fold(a.qx[q], g.Lx), fold(a.qy[q], g.Ly), q, sd[w], si[w], lane);
+        search_one(a, g, fold(a.qx[q], g.Lx), fold(a.qy[q], g.Ly), q, R, est2, sd[w], si[w], lane);
 }
 
 // The nodes that the search by cells left over, one warp each (the warp of
@@ -647,13 +653,27 @@ __global__ void __launch_bounds__(kWarps * 32, 8) leftover_kernel(QueryArgs a) {
     __shared__ unsigned long long sd[kWarps][kCap];
     __shared__ int si[kWarps][kCap];
     const int w = threadIdx.x >> 5, lane = threadIdx.x & 31;
-    const int count = *a.left;
-    if (count == 0) return;
+    const int left = *a.left;
+    if (left == 0) return;
     const Grid g = a.g ? *a.g : a.gv;
-    for (int i = blockIdx.x * kWarps + w; i < count; i += gridDim.x * kWarps) {
+    for (int i = blockIdx.x * kWarps + w; i < left; i += gridDim.x * kWarps) {
         const int t = a.list[i];
         const double2 q = a.sxy[t];
-        search_one(a, g, q.x, q.y, a.sidx[t], sd[w], si[w], lane);
+        // the density around the node, from the 3 x 3 cells (none wrapped)
+        const int row = cell_coord(q.y, g.y0, g.hy, g.cy) - 1 + lane;
+        int count = 0, cells = 0;
+        if (lane < 3 && row >= 0 && row < g.cy) {
+            const int cx = cell_coord(q.x, g.x0, g.hx, g.cx);
+            const int c0 = max(cx - 1, 0), c1 = min(cx + 1, g.cx - 1);
+            count = a.start[row * g.cx + c1 + 1] - a.start[row * g.cx + c0];
+            cells = c1 - c0 + 1;
+        }
+        count = __reduce_add_sync(0xffffffffu, count);
+        cells = __reduce_add_sync(0xffffffffu, cells);
+        const double per = static_cast<double>(count) / cells;
+        const int R = min(rings_at(a.k, g.per),
+                          max(1, (int)ceil(1.15 * sqrt((a.k + 1) / (3.141592653589793 * per)))));
+        search_one(a, g, q.x, q.y, a.sidx[t], R, radius2_at(a.k, g, per), sd[w], si[w], lane);
     }
 }
 

@@ -50,6 +50,8 @@ CASES = [
     (_clusters, 3000, 100, 2.0),  # 6.1 / 1.1: all kept distances in one bucket
     (_square, 200, 128, 2.0),     # 14.5 / 1.1: a circle without a bound
     (_uniform, 200, 100, 2.0),    # 4.8 / 1.2
+    (_graded(1000), 20000, 13, 0.4),  # 0.84 / 0.11: the general search over cells full of nodes
+    (_graded(100), 1000, 13, 1.5),    # 3.5 / 0.68
 ]
 
 
