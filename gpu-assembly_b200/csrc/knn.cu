@@ -369,6 +369,7 @@ struct QueryArgs {
     // (in cell order) that it leaves to leftover_kernel and their number
     int cand_cap, keep_cap;
     int split;  // warps a cell
+    int most;   // queries a warp takes of its cell, the rest is left over
     int* list;
     int* left;
 };
@@ -794,6 +795,14 @@ __device__ __forceinline__ void rank_kept(unsigned long long* kd, int* ki, int* 
     __syncwarp();
 }
 
+// The nodes first + i of the bits i of `which` go to leftover_kernel.
+__device__ __forceinline__ void leave_over(const QueryArgs& a, int first, unsigned which, int lane) {
+    int at = 0;
+    if (lane == 0) at = atomicAdd(a.left, __popc(which));
+    at = __shfl_sync(0xffffffffu, at, 0);
+    if ((which >> lane) & 1u) a.list[at + __popc(which & ((1u << lane) - 1u))] = first + lane;
+}
+
 // One warp per cell, persistent over the cells. The general search spends 1,900
 // warp instructions a query, most of them on comparing every kept candidate
 // with every other; here the candidate block is loaded once a cell and the
@@ -821,7 +830,10 @@ __global__ void __launch_bounds__(kWarps * 32, NSMAX > 5 ? 6 : 8) cell_query_ker
         // this warp's part of the cell's nodes
         const int cell = item / a.split, part = item - cell * a.split;
         const int first = a.start[cell], own = a.start[cell + 1] - first;
-        const int q0 = first + own * part / a.split, q1 = first + own * (part + 1) / a.split;
+        const int q0 = first + own * part / a.split, qe = first + own * (part + 1) / a.split;
+        const int q1 = min(qe, q0 + a.most);
+        for (int qb = q1; qb < qe; qb += 32)
+            leave_over(a, qb, qe - qb >= 32 ? 0xffffffffu : (1u << (qe - qb)) - 1u, lane);
         if (q0 == q1) continue;
         const int ccy = cell / g.cx, ccx = cell - ccy * g.cx;
         for (int qb = q0; qb < q1; qb += 32) {
@@ -991,12 +1003,7 @@ __global__ void __launch_bounds__(kWarps * 32, NSMAX > 5 ? 6 : 8) cell_query_ker
                 pending = failed;
                 ++R;
             }
-            if (pending) {  // what neither block completed
-                int at = 0;
-                if (lane == 0) at = atomicAdd(a.left, __popc(pending));
-                at = __shfl_sync(0xffffffffu, at, 0);
-                if ((pending >> lane) & 1u) a.list[at + __popc(pending & ((1u << lane) - 1u))] = qb + lane;
-            }
+            if (pending) leave_over(a, qb, pending, lane);  // what neither block completed
         }
     }
 }
@@ -1126,13 +1133,25 @@ QueryArgs query_args(const Workspace& w, const Grid* gp, const Grid& gv, int k, 
 }
 
 // The nodes' own stencils over the binned nodes. A small set's cells are shared by
-// several warps, so that all the warps of the chip take part: 3,000 nodes of
-// fourfold varying density, us, one warp a cell and up to eight: k = 21 45 -> 35, k =
-// 35 70 -> 43, k = 61 125 -> 57; of a disk k = 61 70 -> 31. Up to 8,192 nodes about one
-// part a resident warp (two: 3,000 nodes of a square, k = 12, 30 us instead of 26),
-// above them two (25,000 nodes of varying density, k = 61: 110 us, one 163).
-constexpr int kMaxSplit = 8;
+// several warps, as many as the chip holds at once: 3,000 nodes of fourfold varying density,
+// us, one warp a cell and several: k = 21 45 -> 39, k = 35 70 -> 42, k = 61 125 -> 51;
+// periodic, 8,000 nodes, k = 56 three parts (one wave) 46, four 52. Above kSmallNodes about 48
+// parts an SM (25,000 nodes of varying density, k = 61: 110 us, one a cell 163).
+//
+// A cell far above the mean would still leave its warps a long queue while the others
+// are done: a warp takes 2.5 times the mean of a part, and the rest go to
+// leftover_kernel, one warp each (8,000 nodes of thirtyfold varying density, k = 21:
+// 112 -> 60 us; 3,000 nodes in twenty clusters, k = 28: 215 -> 75). In a grid of up to 5 x 5 cells a
+// block is the whole set, and sharing it gains nothing on sets of uneven density: all nodes
+// go there (200 nodes, k = 128, density falling a thousandfold: 181 us by cells, 38).
+//
+// A small set's list of candidates has room for a random set's 5 x 5 cells too (8,000
+// nodes, k = 13: one ring was often too little, 60 -> 51 us).
+constexpr int kMaxSplit = 32;
 cudaError_t enqueue_cells(QueryArgs a, size_t cells, bool periodic, int sms, cudaStream_t st) {
+    const bool small = a.nq <= kSmallNodes;
+    if (small)
+        a.cand_cap = std::min(kMaxCand, std::max(a.cand_cap, static_cast<int>(35.0 * a.nq / cells + 31) / 32 * 32));
     const size_t smem = kWarps * cell_smem(a.cand_cap, a.keep_cap);
     void (*kern)(QueryArgs) = nullptr;
     if (a.keep_cap <= 96)
@@ -1148,8 +1167,12 @@ cudaError_t enqueue_cells(QueryArgs a, size_t cells, bool periodic, int sms, cud
         const cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, most);
         if (e != cudaSuccess) return e;
     }
-    const size_t items = static_cast<size_t>(sms) * (a.nq <= kSmallNodes ? 24 : 48);
+    // resident blocks an SM by the kernel's register bound and its shared memory
+    const size_t per_sm = std::min<size_t>(a.keep_cap > 160 ? 6 : 8, (227 << 10) / (smem + 1024));
+    const size_t items = static_cast<size_t>(sms) * (small ? kWarps * per_sm : 48);
     a.split = static_cast<int>(std::min<size_t>(kMaxSplit, std::max<size_t>(1, items / cells)));
+    const double mean = a.nq / (static_cast<double>(cells) * a.split);
+    a.most = cells <= 25 ? 0 : static_cast<int>(std::ceil(2.5 * mean)) + 1;
     const size_t want = (cells * a.split + kWarps - 1) / kWarps;
     const int blocks = static_cast<int>(std::max<size_t>(1, std::min<size_t>(want, sms * 64)));
     kern<<<blocks, kWarps * 32, smem, st>>>(a);

@@ -52,6 +52,9 @@ CASES = [
     (_uniform, 200, 100, 2.0),    # 4.8 / 1.2
     (_graded(1000), 20000, 13, 0.4),  # 0.84 / 0.11: the general search over cells full of nodes
     (_graded(100), 1000, 13, 1.5),    # 3.5 / 0.68
+    (_clusters, 3000, 28, 2.0),  # 3.8 / 1.2: a few cells hold every node
+    (_clusters, 8000, 64, 1.5),  # 2.3 / 1.0
+    (_layer, 8000, 21, 0.95),    # 1.3 / 0.65
 ]
 
 
