@@ -117,11 +117,13 @@ __device__ __forceinline__ void sts2(double* s, double a, double b) {
 constexpr uint32_t kLow = 123u << 20, kHigh = 1923u << 20;
 constexpr int kMaxExp = 500;
 
-// 1 / a, correctly rounded: an approximation y of at least 20 bits, one
-// third-order step (error below 2^-59 before rounding) and Markstein's final
-// step y + y (1 - a y) (P. Markstein, IA-64 and Elementary Functions, 2000,
-// ch. 8), which rounds correctly for every a whose mantissa is not all ones.
-// For the fast range and a low word other than ~0.
+// 1 / a, correctly rounded, for the fast range and a low word other than ~0. From an
+// approximation y of at least 20 bits, with e = 1 - a y (|e| < 2^-20, to 2^-53 of
+// itself): 1 / a = y / (1 - e) = y (1 + e + e^2 + e^3 + ...). y + y (e + e^2) leaves e^3
+// < 2^-60 and its own rounding: within 1/2 + 2^-7 ulp of 1 / a. The residual 1 - a y
+// of such a y is exact in one fused multiply-add, and Markstein's final step y + y (1 - a y)
+// then rounds correctly for every a whose mantissa is not all ones (P. Markstein, IA-64
+// and Elementary Functions, 2000, ch. 8).
 __device__ __forceinline__ double rcp_fast(double a) {
     double y;
     asm("rcp.approx.ftz.f64 %0, %1;" : "=d"(y) : "d"(a));
@@ -130,10 +132,11 @@ __device__ __forceinline__ double rcp_fast(double a) {
     return fma(y, fma(-a, y, 1.0), y);
 }
 
-// sqrt(a), correctly rounded (same source, ch. 9): g ~ sqrt(a) and h ~
-// 1 / (2 sqrt(a)) from an approximate reciprocal root by one third-order step
-// (r = 1/2 - g h; 1 / sqrt(1 - 2r) = 1 + r + 3/2 r^2 + O(r^3)), then g + h (a -
-// g^2). For the fast range.
+// sqrt(a), correctly rounded, for the fast range (same source, ch. 9). From y ~ 1 /
+// sqrt(a) of at least 20 bits: g = a y, h = y / 2, and r = 1/2 - g h, so that a y^2 = 1 - 2 r
+// and sqrt(a) = g (1 - 2 r)^(-1/2) = g (1 + r + 3/2 r^2 + 5/2 r^3 + ...), likewise 1 / (2
+// sqrt(a)) from h. Two terms leave 5/2 r^3 < 2^-58 and the rounding; the residual a - g^2
+// is exact in one fused multiply-add, and g + h (a - g^2) rounds correctly.
 __device__ __forceinline__ double sqrt_fast(double a) {
     double y;
     asm("rsqrt.approx.ftz.f64 %0, %1;" : "=d"(y) : "d"(a));
