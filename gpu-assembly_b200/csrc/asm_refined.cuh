@@ -578,14 +578,14 @@ __device__ __forceinline__ void assemble(const AsmParams& p, const Item& it, con
     cp_async_wait_all();
     __syncwarp();
     const int ks = it.ks, n = NP + ks, nt = (n + 7) >> 3;
-    const int e = dm::gather_scale<L::KMAX, true, false>(p, it.off, ks, it.x0, it.y0, xy, lane);
+    const int e = dm::gather_scale<L::KMAX, true, false>(p, dm::offset_of(p, it), ks, it.x0, it.y0, xy, lane);
     __syncwarp();
     bool bad = fill_system<L, NRHS, P, Q>(p, S, M, b, xy, ks, e, lane);
     bad = bad || e < -dm::kMaxExp || e > dm::kMaxExp;
     __syncwarp();
     dm::init_order(lists, piv, n, lane);
     if (nx.s >= 0)
-        for (int j = lane; j < nx.ks; j += 32) cp_async4(nja + j, p.ja + nx.off + j);
+        for (int j = lane; j < nx.ks; j += 32) cp_async4(nja + j, p.ja + dm::offset_of(p, nx) + j);
     __syncwarp();
     bad = eliminate<L, NRHS>(S, lists, piv, n, NP, lane) || bad;
     bool failed = __any_sync(ALL, bad);
@@ -660,7 +660,7 @@ __device__ __forceinline__ void assemble(const AsmParams& p, const Item& it, con
     }
     if (!failed && q < NRHS && q < p.nrhs) {
         // rescaled node weights, src/rbf_operators.h:368-375
-        double* dst = out_column(p, q) + it.off;
+        double* dst = out_column(p, q) + dm::offset_of(p, it);
         const int sh = -op_order(p.col_op[q]) * e;
 #pragma unroll
         for (int t = 0; t < NT; ++t) {
