@@ -22,6 +22,7 @@ struct AsmParams {
     const int* ja;  // fixed width: row s at ja + s*k; CSR: ja + ia[s]
     const int* ia;  // nullptr for fixed width
     int k;          // fixed width stencil size
+    int stride;     // entries from a row to the next: k (CSR: 1, a row is its first entry)
     int row_base;   // fixed width: ja, values and info hold rows row_base.. only
     double Lx, Ly;  // periods (<= 0: open axis)
     int scale;

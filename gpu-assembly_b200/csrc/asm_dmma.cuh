@@ -878,10 +878,32 @@ __device__ __forceinline__ bool fill_shape(const AsmParams& p, Sh sh, double* S,
     }
 }
 
+// Stencil s: its row in ja and the value arrays (in CSR form its first entry), its
+// size, its centre.
+struct Item {
+    int s, row, ks;
+    double x0, y0;
+};
+__device__ __forceinline__ Item item_of(const AsmParams& p, int s) {
+    Item it{s, s - p.row_base, p.k, __ldg(p.x + s), __ldg(p.y + s)};
+    if (p.ia) {
+        it.row = __ldg(p.ia + s);
+        it.ks = __ldg(p.ia + s + 1) - it.row;
+    }
+    return it;
+}
+// Its first entry there, in 64 bits: a fixed-width batch may hold more than 2^31. Formed
+// where it is used: carried along it takes registers (600,000 stencils, k = 64: 37.0 ms,
+// this way 36.2, in 32 bits 35.7).
+__device__ __forceinline__ long long offset_of(const AsmParams& p, const Item& it) {
+    return static_cast<long long>(static_cast<unsigned long long>(static_cast<unsigned>(it.row)) *
+                                  static_cast<unsigned>(p.stride));
+}
+
 // The careful path of one stencil, from its global data: everything the fast
 // path leaves out (coincident nodes, zero pivots, extreme magnitudes). Cold.
 template <class L, int NRHS, int NW, class Sh>
-__device__ __noinline__ void assemble_careful(const AsmParams& p, Sh sh, int s, long long off, int ks,
+__device__ __noinline__ void assemble_careful(const AsmParams& p, Sh sh, int s, int row, int ks,
                                               char* base, int warp, int lane) {
     constexpr int LDS = L::LDS;
     double2* xy = reinterpret_cast<double2*>(base + L::off_xy);
@@ -889,6 +911,7 @@ __device__ __noinline__ void assemble_careful(const AsmParams& p, Sh sh, int s, 
     uint8_t* lists = reinterpret_cast<uint8_t*>(base + L::off_list);
     uint8_t* piv = reinterpret_cast<uint8_t*>(base + L::off_piv);
     int* nia = reinterpret_cast<int*>(base + L::off_nia);
+    const long long off = offset_of(p, Item{s, row, ks, 0.0, 0.0});
     const int np = sh.np(), n = np + ks;
     stencil_sync<NW>();
     int e = 0;
@@ -908,27 +931,6 @@ __device__ __noinline__ void assemble_careful(const AsmParams& p, Sh sh, int s, 
         if (lane == 0 && p.info) p.info[s - p.row_base] = info;
     }
     stencil_sync<NW>();
-}
-
-// Stencil s: its row in ja and the value arrays (in CSR form its first entry), its
-// size, its centre.
-struct Item {
-    int s, row, ks;
-    double x0, y0;
-};
-__device__ __forceinline__ Item item_of(const AsmParams& p, int s) {
-    Item it{s, s - p.row_base, p.k, __ldg(p.x + s), __ldg(p.y + s)};
-    if (p.ia) {
-        it.row = __ldg(p.ia + s);
-        it.ks = __ldg(p.ia + s + 1) - it.row;
-    }
-    return it;
-}
-// Its first entry there, in 64 bits: a fixed-width batch may hold more than 2^31. Formed
-// where it is used; carried along it takes registers (150,000 stencils, k = 64: 9.50 ms,
-// this way 9.33, in 32 bits 9.26).
-__device__ __forceinline__ long long offset_of(const AsmParams& p, const Item& it) {
-    return static_cast<long long>(it.row) * (p.ia ? 1 : p.k);
 }
 
 // The neighbour coordinates of stencil nx and its centre, asynchronously, by
@@ -1011,7 +1013,7 @@ __device__ __forceinline__ void assemble(const AsmParams& p, Sh sh, const Item& 
     }
     if (bad) {
         if constexpr (SHARED) cp_async_wait_all();
-        assemble_careful<L, NRHS, NW>(p, sh, it.s, offset_of(p, it), ks, base, warp, lane);
+        assemble_careful<L, NRHS, NW>(p, sh, it.s, it.row, ks, base, warp, lane);
         if (SHARED && fetcher && nx.s >= 0) fetch_nodes<L, false>(p, nx, base, lane);
         return;
     }

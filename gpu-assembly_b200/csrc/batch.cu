@@ -330,6 +330,7 @@ int rbfb_assemble_csr(rbfb_ctx* ctx, const rbfb_desc* desc, int nstencils, const
     p.y = y;
     p.ja = ja;
     p.ia = ia;
+    p.stride = 1;
     p.Lx = desc->period[0];
     p.Ly = desc->period[1];
     p.scale = desc->scale;

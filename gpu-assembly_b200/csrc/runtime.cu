@@ -249,6 +249,7 @@ int enqueue_fixed(rbfb_ctx* ctx, const rbfb_desc* desc, int first, int count, co
     if (p.nrhs > variants()[v].nrhs)
         return fail(ctx, RBFB_EUNSUPPORTED, "more right-hand sides than the compiled kernels hold");
     p.k = k;
+    p.stride = k;
     p.item_base = first;
     p.row_base = row_base;
     if (count == 0) return RBFB_OK;
