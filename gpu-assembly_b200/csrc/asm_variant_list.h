@@ -12,12 +12,11 @@
 // k = 64 two warps a stencil 4.09, four 4.13.
 //
 // RBFB_IR_VARIANT(name, NMAX, NRHS, P, Q, GPB, MINB): the refined form
-// (asm_refined.cuh), one warp a stencil, GPB stencils a CTA. Same counts, ms
-// (the former one-warp kernel and register kernels in brackets): k = 35 five
-// stencils a CTA 6.40, ten 6.44, two 6.53, three (9 resident) 7.17, one 7.37
-// [12.27]; k = 38 nine 7.28, three 7.49; k = 21 four 2.17, one 2.19 [4.07];
-// k = 45, degree 4 6.63 in the 64 class, 10.46 in the 80 class [11.88]; k = 64
-// 14.5 [24.9], of which the FP64 kernel takes 4.1 (it redoes nearly all).
+// (asm_refined.cuh), one warp a stencil, GPB stencils a CTA. Same counts, ms:
+// k = 35 five stencils a CTA 6.40, ten 6.44, two 6.53, three (9 resident) 7.17, one
+// 7.37; k = 38 nine 7.28, three 7.49; k = 21 four 2.17, one 2.19; k = 45, degree 4
+// 6.63 in the 64 class, 10.46 in the 80 class; k = 64 14.5, of which the FP64 kernel
+// takes 4.1 (it redoes nearly all).
 RBFB_DM_VARIANT(b64_p2q3_n32_w1x1, 32, 3, 2, 3, 1, 1, 20)
 RBFB_DM_VARIANT(b64_p2q3_n32_w1x4_r8, 32, 8, 2, 3, 1, 4, 4)
 RBFB_DM_VARIANT(b64_p3q5_n45_w1x3, 45, 3, 3, 5, 1, 3, 4)

@@ -648,8 +648,10 @@ __global__ void __launch_bounds__(kWarps * 32, 8) query_kernel(QueryArgs a) {
 
 // The nodes that the search by cells left over, one warp each (the warp of
 // their cell would take them one after another: 11,359 nodes of fourfold varying
-// density, k = 61: 261 -> 141 us; 60,000 of a disk 331 -> 252). The launch costs a
-// set that leaves none 2 us.
+// density, k = 61: 261 us, this way 81). Its cells are the large ones of the search by
+// cells, so it starts from the density around each node, not from the mean (20,000 nodes,
+// density falling a thousandfold, k = 13: 3.5 ms from the mean, 0.16). The launch costs a set that
+// leaves none 2 us.
 __global__ void __launch_bounds__(kWarps * 32, 8) leftover_kernel(QueryArgs a) {
     __shared__ unsigned long long sd[kWarps][kCap];
     __shared__ int si[kWarps][kCap];
@@ -803,12 +805,12 @@ __device__ __forceinline__ void leave_over(const QueryArgs& a, int first, unsign
     if ((which >> lane) & 1u) a.list[at + __popc(which & ((1u << lane) - 1u))] = first + lane;
 }
 
-// One warp per cell, persistent over the cells. The general search spends 1,900
-// warp instructions a query, most of them on comparing every kept candidate
+// One warp per cell (small sets: several), persistent over the cells. The general search
+// spends 1,900 warp instructions a query, most of them on comparing every kept candidate
 // with every other; here the candidate block is loaded once a cell and the
-// ranking is linear in the kept ones: about 460 a query at k = 21. Bound by
-// instruction issue (72 % of the issue slots at 27 warps per SM). 1M nodes of
-// a disk, k = 21: 2.23 -> 0.54 ms; 1M periodic, k = 35: 2.60 -> 0.95 ms.
+// ranking is linear in the kept ones: 530 a query at k = 21, 690 at k = 35. Bound by
+// instruction issue (74 % of the issue slots at 27 warps per SM). The whole search, 1M nodes of
+// a disk, k = 21: 2.24 ms by the general one, 0.52; 1M periodic, k = 35: 2.48, 0.85.
 // NSMAX: kept entries a lane at most (keep_cap / 32); bounded to 8 CTAs (32
 // warps, 64 registers) per SM, 6 for the largest lists.
 template <bool PERIODIC, int NSMAX>
@@ -901,7 +903,8 @@ __global__ void __launch_bounds__(kWarps * 32, NSMAX > 5 ? 6 : 8) cell_query_ker
                 }
                 const int total = __shfl_sync(0xffffffffu, incl, 15);
                 const float area = static_cast<float>(nrows * (xhi - xlo + 1));
-                // a dense block: one ring is enough for k
+                // a dense block (by the list's capacity, at the plane's border also by its
+                // density): one ring is mostly enough for k
                 if (R == 2 && !shrunk && (total > a.cand_cap || total * 3.1416f > 1.6f * (k + 1) * area)) {
                     shrunk = true;
                     R = 1;
@@ -1055,16 +1058,15 @@ int ensure_ws(rbfb_ctx* ctx, size_t n, size_t cells) {
     return RBFB_OK;
 }
 
-// Mean nodes per cell. For the nodes' own stencils the circle of two cells'
-// radius (4 pi cells), inside every 5 x 5 block, has to hold k nodes also where
-// the density is about half the mean; larger cells also share a block between
-// more queries. Measured for (k + 4 sqrt k) / 12.6, 10, 8, 7 nodes a cell: 631,
-// 614, 728, 537 us (1M disk, k = 21), 891, 911, 951, 973 (1M periodic, k =
-// 35), 1542, 773, 732, 676 (300k nodes of fourfold varying density, k = 64).
+// Mean nodes per cell. For the nodes' own stencils: larger cells share a block between
+// more queries, but a block above the list's capacity (6.5 (k + 1)) falls back from two
+// rings to one, in which not every query finds k. Measured for (k + 4 sqrt k) / 12.6, 10, 8, 7
+// nodes a cell: 631, 614, 728, 537 us (1M disk, k = 21: a disk fills its box to 0.79, so at /
+// 7 most cells take one ring), 891, 911, 951, 973 (1M periodic, k = 35), 1542, 773, 732, 676
+// (300k nodes of fourfold varying density, k = 64).
 // A small set takes smaller cells, towards a cell for every resident warp, down to
 // 1.3 times what two rings need for k (1.0 times leaves many nodes of a varying
-// density over: 11,359 nodes, k = 61, 226 us against 106).
-// Arbitrary query points: kPerCell.
+// density over). Arbitrary query points: kPerCell.
 double per_cell(int k, int n, int sms, bool own) {
     if (!own) return kPerCell;
     const double root = std::sqrt(static_cast<double>(k));

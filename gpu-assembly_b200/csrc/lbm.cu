@@ -264,10 +264,9 @@ __device__ __forceinline__ void copy_slab(V* dst, const V* src, int m, const Pie
 // KT > 0 fixes k at compile time: the index rows land in the second weight slab
 // and each lane keeps its own in registers for the tile, which saves the index
 // slab and its reads, and the gathers of a row are in flight at once.
-// 1M nodes (100k), FP64, us: k = 15 264 -> 188 (42 -> 22), k = 18 361 -> 218 (47
-// -> 27), k = 21 265 -> 248 (37 -> 31), k = 24 589 -> 312 (64 -> 38); 6.4 TB/s at
-// k = 21. Before, even k was copied entry by entry and the sizes other than 21 read
-// their indices from a slab for every direction.
+// 1M nodes (100k), FP64, us, in the general kernel and in that of the size: k = 15 264
+// and 188 (42, 22), k = 18 361 and 218 (47, 27), k = 24 589 and 312 (64, 38); k = 21 259 us, 6.46
+// TB/s, with the two fields in turn. A size has its kernel where 16-byte copies can be: n k even.
 // Resident CTAs that the registers are cut for: those that the slabs allow, at
 // most 6 for short rows and 4 (128 registers) from 16 entries on, where more
 // gathers in flight are worth more than more warps. 1M nodes, k = 15 187 (6) and
@@ -395,7 +394,8 @@ int launch_stream_collide(int n, int k, const int* ja, const double* W, T omega,
     return cudaGetLastError() == cudaSuccess ? RBFB_OK : RBFB_ECUDA;
 }
 
-// A kernel for each stencil size up to kMaxFixed, from kMinFixed (degree 1) on.
+// A kernel for each stencil size up to kMaxFixed, from kMinFixed (degree 1) on, for
+// aligned arrays and an even n k (every direction's weights then start on a 16-byte boundary).
 constexpr int kMinFixed = 5, kMaxFixed = 32;
 template <typename T, int KT, class... A>
 int launch_fixed(int n, int k, A... args) {

@@ -15,9 +15,11 @@
 // The iteration streams memory, so HBM bandwidth is its roofline: each step
 // reads the operator (12 B per stored weight, twice) and a handful of
 // vectors. What holds the operator passes below it is the latency of their
-// gathers (one per stored weight), which each thread hides by summing its
-// own row in row order with eight gathers in flight (row_sum.cuh). It is
-// laid out as five kernels per iteration, each one pass over the rows:
+// gathers (one per stored weight), of which each thread keeps eight in flight:
+// it sums its own row, staged in shared memory or walked in global memory
+// (walk_rows). Systems that fit L2 are bound by the chain of the kernels
+// themselves: each may start while its predecessor ends. It is laid out as
+// five kernels per iteration, each one pass over the rows:
 //   p_kernel       p = r + beta (p - omega v)
 //   spmv_v_kernel  v = A p, with the partial sums of (rh, v)
 //   s_kernel       s = r - alpha v
@@ -25,12 +27,17 @@
 //   update_kernel  u += alpha p + omega s, r = s - omega t, with (rh, r), (r, r)
 // s gets a pass of its own so that A s gathers one vector per stored weight
 // rather than forming s from two gathered ones (r and v).
-// The scalars live in device memory: the block that finishes a kernel last
-// (an atomic arrival count, no waiting) adds the blocks' partial sums in
-// block order and computes the next coefficients and the stop flag, which
-// every later kernel reads at entry. The host only looks at the flag once
-// per chunk of kChunk iterations, which run as one CUDA graph on a
-// non-default stream.
+// The scalars live in device memory. The partial sums of an operator pass are
+// added, in block order, by every block of the next kernel for itself: those of s_kernel
+// form (rh, v) and alpha, those of update_kernel (t, s), (t, t), (s, s) and omega. Only
+// the sums of update_kernel (and of the initial residual) are added by the block that
+// finishes last (an atomic arrival count, no waiting), which computes the next
+// coefficients and the stop flag that every later kernel reads at entry. Each kernel
+// waits for its predecessor before it touches anything that one touches, and lets its
+// successor start only after that wait: when a kernel writes, everything before its
+// predecessor has ended too (the partial sums are written again by the kernel after
+// the one that reads them). The host only looks at the flag once per chunk of kChunk
+// iterations, which run as one CUDA graph on a non-default stream.
 //
 // Every sum has a fixed order, so results are reproducible and the CPU
 // oracle follows them exactly: rows in fused multiply-adds from zero; a
@@ -55,11 +62,11 @@ namespace solve {
 constexpr int kThreads = 256;
 constexpr int kWarps = kThreads / 32;
 constexpr int kChunk = 8;  // iterations between two looks at the stop flag
-// Blocks per SM that stay resident together (at most 40 registers a
-// thread); the grid is that many per SM, so none waits for a second wave.
+// Blocks of the grid per SM (the fixed order of the sums follows from it). They are
+// resident together in init_kernel alone, at 40 registers a thread.
 constexpr int kBlocksPerSm = 6;
-// The vector passes hold four rows' operands in flight: fewer blocks, more
-// registers.
+// The vector passes hold four rows' operands in flight: 64 and 80 registers, so that
+// four and three blocks per SM are resident, the grid in two waves.
 constexpr int kVectorBlocksPerSm = 4, kUpdateBlocksPerSm = 3;
 // The operator passes stage each warp's rows (its entries in one piece, up to
 // kStageEntries; 32 rows, or 16 at a time) in shared memory: 96 KB a block, two

@@ -22,8 +22,9 @@ namespace rbfb {
 // under an L2 evict-first policy, and each lane sums its own row from there,
 // eight gathers of u in flight. A thread-per-row walk of global memory touches a
 // line per lane and load: 1.6 GB through the L1s for 437 MB of operator, and the
-// L1 bound it. 16 rows a warp leave room for 32 warps per SM. 1M rows, k = 35:
-// 128 -> 79 us (5.5 TB/s of the operator's bytes); 32 rows a warp, 16 warps: 92.
+// L1 bound it. 16 rows a warp leave room for 32 warps per SM. 1M rows, k = 35, the
+// operator from HBM: 131 us by a thread a row, 94 so (4.5 TB/s of its bytes); again and again, what
+// is in L2 of it, 128 and 83, with 32 rows and 16 warps 92.
 // k a multiple of 4 would put the rows of all lanes on a few banks: their rows
 // are padded by a 16-byte piece (PAD; 60,000 rows, k = 36: 9.9 us, 10.0 walked).
 constexpr int kSpmvWarps = 4, kTileRows = 16;
