@@ -555,7 +555,7 @@ __device__ __forceinline__ void search_one(const QueryArgs& a, const Grid& g, do
         }
         if (total < k) {
             if (reach < bound2) {  // same block, a wider radius, then the full bound
-                reach = reach > est2 ? INFINITY : 4.0 * est2;
+                reach = reach == est2 && est2 > 0.0 ? 4.0 * est2 : INFINITY;
                 continue;
             }
             R += max(1, R / 2);

@@ -5,7 +5,7 @@ cells once took on them and what it takes."""
 import numpy as np
 import pytest
 
-import rbf_b200 as R
+import oracle as O
 from rbf_b200 import nodesets as NS
 
 pytestmark = pytest.mark.gpu
@@ -82,3 +82,16 @@ def test_search_against_the_general_one(ctx, torch_cuda, nodes, n, k, multiple):
     ratio = sorted(_us(T, lambda: ctx.knn_stencils(x, y, k, ja)) /
                    _us(T, lambda: ctx.knn_query(x, y, x, y, k, want)) for _ in range(3))[1]
     assert ratio < multiple
+
+
+@pytest.mark.parametrize("scale", [1e-170, 1e-155, 1e150])
+def test_extreme_scales_complete(ctx, torch_cuda, scale):
+    """Squared distances, and with them the first radius, that underflow to zero, are
+    subnormal or near the largest double: the search still finishes, ties by index."""
+    T = torch_cuda
+    n, k = 700, 24
+    x, y = (np.ascontiguousarray(a) * scale for a in _uniform(n))
+    ja = T.empty(n * k, dtype=T.int32, device="cuda")
+    ctx.knn_stencils(T.as_tensor(x).cuda(), T.as_tensor(y).cuda(), k, ja)
+    assert ctx.knn_status() == 0
+    np.testing.assert_array_equal(ja.cpu().numpy(), O.knn_brute(x, y, k))
